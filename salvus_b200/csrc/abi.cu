@@ -761,7 +761,8 @@ static int launch_coupling(salvus_problem *p) {
   if (m->physics != SALVUS_COUPLED2D || m->n_cpl == 0) return SALVUS_OK;
   const real *coef = sizeof(real) == 4 ? (const real *)m->d_cpl32.ptr : (const real *)m->d_cpl64.ptr;
   coupling_kernel<real><<<blocks_for(m->n_cpl, 256), 256, 0, p->stream>>>(
-      m->n_cpl_fluid, m->n_cpl, m->d_cpl_pts.as<int32_t>(), coef, F<real>(p->d_v), F<real>(p->d_r));
+      m->n_cpl_fluid, m->n_cpl, m->d_cpl_pts.as<int32_t>(), coef, F<real>(p->d_v),
+      F<real>(p->d_ap), (real)(0.5 * p->dt), F<real>(p->d_r));
   g_launches++;
   return check_launch("coupling");
 }
@@ -875,7 +876,7 @@ static int launch_fused_interior(salvus_problem *p, const HexInteriorUpdate &iu)
   return fail(SALVUS_E_UNSUPPORTED, "fused hexahedron step: order %d", m->order);
 }
 
-static int step_fused_hex_interior(salvus_problem *p) {
+static int step_fused_hex_interior(salvus_problem *p, bool store_a) {
   const salvus_mesh *m = p->mesh;
   int rc;
   // this stiffness launch writes u (interior nodes): the previous step's
@@ -885,8 +886,8 @@ static int step_fused_hex_interior(salvus_problem *p) {
     ProfScope ps(p, K_STIFF);
     HexInteriorUpdate iu{};
     iu.mi = m->d_mi32.as<float>();
-    iu.v = F<float>(p->d_v);
-    iu.ap = F<float>(p->d_ap);
+    iu.w = F<float>(p->d_v);
+    iu.ap = store_a ? F<float>(p->d_ap) : nullptr;
     iu.dt = (float)p->dt;
     iu.nsrc_elem = p->n_src_uelem;
     iu.src_elem = p->d_src_uelem.as<int64_t>();
@@ -902,8 +903,8 @@ static int step_fused_hex_interior(salvus_problem *p) {
           (int)p->srcs.size(), m->P, p->d_src_elem.as<int64_t>(), p->d_src_par.as<double>(),
           p->d_src_wts.as<double>(), p->d_step.as<int64_t>(), p->dt, F<float>(p->d_r),
           p->n_src_uelem, p->d_src_uelem.as<int64_t>(), m->d_conn.as<int32_t>(),
-          m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v), F<float>(p->d_ap),
-          (float)p->dt);
+          m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v),
+          store_a ? F<float>(p->d_ap) : nullptr, (float)p->dt);
     };
     switch (m->order) {
       case 2: go(std::integral_constant<int, 2>{}); break;
@@ -921,19 +922,21 @@ static int step_fused_hex_interior(salvus_problem *p) {
     gather_list_kernel<float, 3, 0><<<blocks_for(m->n_gnodes, 256), 256, 0, p->stream>>>(
         m->n_gnodes, m->d_gnodes.as<int32_t>(), m->d_inc_off.as<int32_t>(),
         m->d_inc_idx.as<int32_t>(), F<float>(p->d_r), m->d_mi32.as<float>(), F<float>(p->d_u),
-        F<float>(p->d_v), F<float>(p->d_ap), F<float>(p->d_a), (float)p->dt);
+        F<float>(p->d_v), store_a ? F<float>(p->d_ap) : nullptr, nullptr, (float)p->dt);
     g_launches++;
     if ((rc = check_launch("gather update (shared nodes)"))) return rc;
   }
   return launch_receivers<float, 3>(p);
 }
 
+// store_a: keep this step's a in a_ (every step that a caller can see; the
+// steps inside a run only where the fluid-solid coupling reads v)
 template <typename real, int C>
-static int step_fused_t(salvus_problem *p) {
+static int step_fused_t(salvus_problem *p, bool store_a) {
   const salvus_mesh *m = p->mesh;
   int rc;
   if constexpr (std::is_same<real, float>::value && C == 3) {
-    if (hex_interior_fusion(p)) return step_fused_hex_interior(p);
+    if (hex_interior_fusion(p)) return step_fused_hex_interior(p, store_a);
   }
   {
     ProfScope ps(p, K_STIFF);
@@ -952,7 +955,8 @@ static int step_fused_t(salvus_problem *p) {
     constexpr int kGatherThreads = 128;
     gather_kernel<real, C, 0><<<blocks_for(m->G, kGatherThreads), kGatherThreads, 0, p->stream>>>(
         m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<real>(p->d_r),
-        inv_mass<real>(p), F<real>(p->d_u), F<real>(p->d_v), F<real>(p->d_ap), F<real>(p->d_a),
+        inv_mass<real>(p), F<real>(p->d_u), F<real>(p->d_v),
+        store_a || m->physics == SALVUS_COUPLED2D ? F<real>(p->d_ap) : nullptr, nullptr,
         (real)p->dt);
     g_launches++;
     if ((rc = check_launch("gather update"))) return rc;
@@ -1194,12 +1198,32 @@ static int step_batched(salvus_problem *p) {
   return check_launch("batched receivers");
 }
 
-static int step_fused(salvus_problem *p) {
+static int step_fused(salvus_problem *p, bool store_a) {
   if (p->shots > 1) return step_batched(p);
   return by_components(p->c, [&](auto cc) {
     constexpr int C = decltype(cc)::value;
-    return p->prec == SALVUS_FP32 ? step_fused_t<float, C>(p) : step_fused_t<double, C>(p);
+    return p->prec == SALVUS_FP32 ? step_fused_t<float, C>(p, store_a)
+                                  : step_fused_t<double, C>(p, store_a);
   });
+}
+
+// Puts d_v into the form the caller needs: half = true before steps (w = v +
+// dt/2 a_), false before v or a_ is overwritten or dt changes.  One pass over
+// the field, and only when the form changes: a run after a run converts
+// nothing.  Batched problems hold w throughout.
+static int velocity_form(salvus_problem *p, bool half) {
+  if (p->shots > 1 || p->half_step == half) return SALVUS_OK;
+  const int64_t N = p->mesh->G * p->c;
+  const double s = (half ? 0.5 : -0.5) * p->dt;
+  if (p->prec == SALVUS_FP32)
+    axpy_kernel<float><<<blocks_for(N, 256), 256, 0, p->stream>>>(N, (float)s, F<float>(p->d_ap),
+                                                                  F<float>(p->d_v));
+  else
+    axpy_kernel<double><<<blocks_for(N, 256), 256, 0, p->stream>>>(N, s, F<double>(p->d_ap),
+                                                                   F<double>(p->d_v));
+  g_launches++;
+  p->half_step = half;
+  return check_launch("velocity form");
 }
 
 template <typename real, int C>
@@ -1339,8 +1363,8 @@ static int launch_finite_check(salvus_problem *p) {
 // Hexahedron autotuner (FP32 elastic meshes of parallelepipeds, one shot):
 // times the plain step (stiffness, node gather/update) and, where the fused
 // interior form is admissible, that form, each with CTAs of 128 / (N+1)^2
-// elements and with twice as many, on zeroed scratch copies of u, v, a_ and
-// a, and keeps the fastest.  All of them give bitwise the same wavefield
+// elements and with twice as many, on zeroed scratch copies of u and w, and
+// keeps the fastest.  All of them give bitwise the same wavefield
 // (the same arithmetic per element and per node, in the same order), so the
 // choice changes only the time.  Results are cached per (order, elements,
 // nodes, anisotropy, admissible forms, device) for the process; the CTA
@@ -1387,21 +1411,17 @@ static int tune_hex(salvus_problem *p) {
   }
   p->hex_form = 0;
   const size_t nf = (size_t)m->G * 3 * sizeof(float);
-  DeviceBuffer su, sv, sap, sa;
+  DeviceBuffer su, sv;
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < 4 * nf + (size_t(1) << 30) ||
-      su.alloc(nf) || sv.alloc(nf) || sap.alloc(nf) || sa.alloc(nf)) {
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < 2 * nf + (size_t(1) << 30) ||
+      su.alloc(nf) || sv.alloc(nf)) {
     cudaGetLastError();
     return SALVUS_OK;
   }
   SALVUS_CUDA(cudaMemsetAsync(su.ptr, 0, nf, p->stream));
   SALVUS_CUDA(cudaMemsetAsync(sv.ptr, 0, nf, p->stream));
-  SALVUS_CUDA(cudaMemsetAsync(sap.ptr, 0, nf, p->stream));
-  SALVUS_CUDA(cudaMemsetAsync(sa.ptr, 0, nf, p->stream));
   std::swap(p->d_u.ptr, su.ptr);
   std::swap(p->d_v.ptr, sv.ptr);
-  std::swap(p->d_ap.ptr, sap.ptr);
-  std::swap(p->d_a.ptr, sa.ptr);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -1415,20 +1435,18 @@ static int tune_hex(salvus_problem *p) {
         return r;
       gather_kernel<float, 3, 0><<<blocks_for(m->G, 256), 256, 0, p->stream>>>(
           m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<float>(p->d_r),
-          m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v), F<float>(p->d_ap),
-          F<float>(p->d_a), (float)p->dt);
+          m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v), nullptr, nullptr, (float)p->dt);
     } else {
       HexInteriorUpdate iu{};
       iu.mi = m->d_mi32.as<float>();
-      iu.v = F<float>(p->d_v);
-      iu.ap = F<float>(p->d_ap);
+      iu.w = F<float>(p->d_v);
       iu.dt = (float)p->dt;
       if ((r = m->ti ? launch_fused_interior<true>(p, iu) : launch_fused_interior<false>(p, iu)))
         return r;
       gather_list_kernel<float, 3, 0><<<blocks_for(m->n_gnodes, 256), 256, 0, p->stream>>>(
           m->n_gnodes, m->d_gnodes.as<int32_t>(), m->d_inc_off.as<int32_t>(),
           m->d_inc_idx.as<int32_t>(), F<float>(p->d_r), m->d_mi32.as<float>(), F<float>(p->d_u),
-          F<float>(p->d_v), F<float>(p->d_ap), F<float>(p->d_a), (float)p->dt);
+          F<float>(p->d_v), nullptr, nullptr, (float)p->dt);
     }
     g_launches++;
     return check_launch("hexahedron autotuner");
@@ -1459,8 +1477,6 @@ static int tune_hex(salvus_problem *p) {
   cudaStreamSynchronize(p->stream);
   std::swap(p->d_u.ptr, su.ptr);
   std::swap(p->d_v.ptr, sv.ptr);
-  std::swap(p->d_ap.ptr, sap.ptr);
-  std::swap(p->d_a.ptr, sa.ptr);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   m->hex_wide = bw;
@@ -1580,7 +1596,7 @@ static int group_upload(salvus::DeviceBuffer &b, const void *src, size_t bytes, 
   return SALVUS_OK;
 }
 
-static int group_partitioned(salvus_group *g, bool launch);
+static int group_partitioned(salvus_group *g, bool launch, bool store_a);
 
 static int group_fill(salvus_group *g) {
   int64_t bs = 0, bg = 0, br = 0;
@@ -1600,9 +1616,8 @@ static int group_fill(salvus_group *g) {
     s.E = m->E;
     s.G = m->G;
     s.u = p->d_u.as<float>();
-    s.v = p->d_v.as<float>();
+    s.w = p->d_v.as<float>();
     s.ap = p->d_ap.as<float>();
-    s.a = p->d_a.as<float>();
     s.r = p->d_r.as<float>();
     s.dt = (float)p->dt;
     s.dtd = p->dt;
@@ -1676,12 +1691,12 @@ static int group_fill(salvus_group *g) {
     SALVUS_CUDA(cudaMemsetAsync(g->d_sync.ptr, 0, sizeof(GroupSync), g->stream));
   }
   // the partitioned step's CTA ranges and counters (allocated here, before any capture)
-  if (g->partitioned) return group_partitioned(g, false);
+  if (g->partitioned) return group_partitioned(g, false, false);
   return SALVUS_OK;
 }
 
 template <int N, bool kHex, int C>
-static int group_persistent_t(salvus_group *g) {
+static int group_persistent_t(salvus_group *g, bool store_a) {
   constexpr int threads = 128;
   size_t smem = 0;
   if constexpr (kHex) {
@@ -1699,34 +1714,34 @@ static int group_persistent_t(salvus_group *g) {
   kern<<<grid, threads, smem, g->stream>>>(
       g->d_slots.as<GroupSlot>(), g->d_counts.as<GroupCounts>(), (int)g->members.size(),
       g->d_work.as<GroupWork>(), g->total, g->d_done.as<int32_t>(), g->d_sync.as<GroupSync>(),
-      dmatrix<float>(g->m0->basis), g->m0->P, g->wait_limit);
+      dmatrix<float>(g->m0->basis), g->m0->P, g->wait_limit, store_a);
   g_launches++;
   return check_launch("group persistent step");
 }
 
-static int group_persistent(salvus_group *g) {
+static int group_persistent(salvus_group *g, bool store_a) {
   const salvus_mesh *m = g->m0;
   if (m->shape == SALVUS_HEX) {
     switch (m->order) {
-      case 1: return group_persistent_t<1, true, 3>(g);
-      case 2: return group_persistent_t<2, true, 3>(g);
-      case 3: return group_persistent_t<3, true, 3>(g);
-      case 4: return group_persistent_t<4, true, 3>(g);
-      case 5: return group_persistent_t<5, true, 3>(g);
-      case 6: return group_persistent_t<6, true, 3>(g);
+      case 1: return group_persistent_t<1, true, 3>(g, store_a);
+      case 2: return group_persistent_t<2, true, 3>(g, store_a);
+      case 3: return group_persistent_t<3, true, 3>(g, store_a);
+      case 4: return group_persistent_t<4, true, 3>(g, store_a);
+      case 5: return group_persistent_t<5, true, 3>(g, store_a);
+      case 6: return group_persistent_t<6, true, 3>(g, store_a);
     }
   } else {
     switch (m->order) {
-      case 1: return group_persistent_t<1, false, 1>(g);
-      case 2: return group_persistent_t<2, false, 1>(g);
-      case 3: return group_persistent_t<3, false, 1>(g);
-      case 4: return group_persistent_t<4, false, 1>(g);
-      case 5: return group_persistent_t<5, false, 1>(g);
-      case 6: return group_persistent_t<6, false, 1>(g);
-      case 7: return group_persistent_t<7, false, 1>(g);
-      case 8: return group_persistent_t<8, false, 1>(g);
-      case 9: return group_persistent_t<9, false, 1>(g);
-      case 10: return group_persistent_t<10, false, 1>(g);
+      case 1: return group_persistent_t<1, false, 1>(g, store_a);
+      case 2: return group_persistent_t<2, false, 1>(g, store_a);
+      case 3: return group_persistent_t<3, false, 1>(g, store_a);
+      case 4: return group_persistent_t<4, false, 1>(g, store_a);
+      case 5: return group_persistent_t<5, false, 1>(g, store_a);
+      case 6: return group_persistent_t<6, false, 1>(g, store_a);
+      case 7: return group_persistent_t<7, false, 1>(g, store_a);
+      case 8: return group_persistent_t<8, false, 1>(g, store_a);
+      case 9: return group_persistent_t<9, false, 1>(g, store_a);
+      case 10: return group_persistent_t<10, false, 1>(g, store_a);
     }
   }
   return fail(SALVUS_E_UNSUPPORTED, "no grouped step for order %d", m->order);
@@ -1735,7 +1750,7 @@ static int group_persistent(salvus_group *g) {
 // launch=false: size the member CTA ranges (once) and allocate their counters;
 // launch=true: one cooperative launch of the step
 template <int N, bool kHex, int C>
-static int group_partitioned_t(salvus_group *g, bool launch) {
+static int group_partitioned_t(salvus_group *g, bool launch, bool store_a) {
   constexpr int threads = 128;
   size_t smem = 0;
   if constexpr (kHex) {
@@ -1798,42 +1813,43 @@ static int group_partitioned_t(salvus_group *g, bool launch) {
                                  (const GroupPart *)g->d_parts.as<GroupPart>(), J,
                                  g->d_bars.as<GroupBar>(), g->d_sync.as<GroupSync>(),
                                  dmatrix<float>(g->m0->basis), g->m0->P,
-                                 (long long)g->wait_limit));
+                                 (long long)g->wait_limit, store_a));
   g_launches++;
   return check_launch("group partitioned step");
 }
 
-static int group_partitioned(salvus_group *g, bool launch) {
+static int group_partitioned(salvus_group *g, bool launch, bool store_a) {
   const salvus_mesh *m = g->m0;
   if (m->shape == SALVUS_HEX) {
     switch (m->order) {
-      case 1: return group_partitioned_t<1, true, 3>(g, launch);
-      case 2: return group_partitioned_t<2, true, 3>(g, launch);
-      case 3: return group_partitioned_t<3, true, 3>(g, launch);
-      case 4: return group_partitioned_t<4, true, 3>(g, launch);
-      case 5: return group_partitioned_t<5, true, 3>(g, launch);
-      case 6: return group_partitioned_t<6, true, 3>(g, launch);
+      case 1: return group_partitioned_t<1, true, 3>(g, launch, store_a);
+      case 2: return group_partitioned_t<2, true, 3>(g, launch, store_a);
+      case 3: return group_partitioned_t<3, true, 3>(g, launch, store_a);
+      case 4: return group_partitioned_t<4, true, 3>(g, launch, store_a);
+      case 5: return group_partitioned_t<5, true, 3>(g, launch, store_a);
+      case 6: return group_partitioned_t<6, true, 3>(g, launch, store_a);
     }
   } else {
     switch (m->order) {
-      case 1: return group_partitioned_t<1, false, 1>(g, launch);
-      case 2: return group_partitioned_t<2, false, 1>(g, launch);
-      case 3: return group_partitioned_t<3, false, 1>(g, launch);
-      case 4: return group_partitioned_t<4, false, 1>(g, launch);
-      case 5: return group_partitioned_t<5, false, 1>(g, launch);
-      case 6: return group_partitioned_t<6, false, 1>(g, launch);
-      case 7: return group_partitioned_t<7, false, 1>(g, launch);
-      case 8: return group_partitioned_t<8, false, 1>(g, launch);
-      case 9: return group_partitioned_t<9, false, 1>(g, launch);
-      case 10: return group_partitioned_t<10, false, 1>(g, launch);
+      case 1: return group_partitioned_t<1, false, 1>(g, launch, store_a);
+      case 2: return group_partitioned_t<2, false, 1>(g, launch, store_a);
+      case 3: return group_partitioned_t<3, false, 1>(g, launch, store_a);
+      case 4: return group_partitioned_t<4, false, 1>(g, launch, store_a);
+      case 5: return group_partitioned_t<5, false, 1>(g, launch, store_a);
+      case 6: return group_partitioned_t<6, false, 1>(g, launch, store_a);
+      case 7: return group_partitioned_t<7, false, 1>(g, launch, store_a);
+      case 8: return group_partitioned_t<8, false, 1>(g, launch, store_a);
+      case 9: return group_partitioned_t<9, false, 1>(g, launch, store_a);
+      case 10: return group_partitioned_t<10, false, 1>(g, launch, store_a);
     }
   }
   return fail(SALVUS_E_UNSUPPORTED, "no grouped step for order %d", m->order);
 }
 
-static int group_step(salvus_group *g) {
-  if (g->partitioned) return group_partitioned(g, true);
-  if (!g->stages) return group_persistent(g);
+// store_a: keep a_ (the last step of a run, see step_fused_t)
+static int group_step(salvus_group *g, bool store_a) {
+  if (g->partitioned) return group_partitioned(g, true, store_a);
+  if (!g->stages) return group_persistent(g, store_a);
   const int J = (int)g->members.size();
   const int P = g->m0->P;
   const GroupSlot *slots = g->d_slots.as<GroupSlot>();
@@ -1842,8 +1858,8 @@ static int group_step(salvus_group *g) {
   if ((rc = group_stiffness(g->m0, slots, own, g->n_stiff, g->stream))) return rc;
   if (g->c == 1) group_source<1><<<J, 256, 0, g->stream>>>(slots, P);
   else group_source<3><<<J, 256, 0, g->stream>>>(slots, P);
-  if (g->c == 1) group_gather_update<1><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff);
-  else group_gather_update<3><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff);
+  if (g->c == 1) group_gather_update<1><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff, store_a);
+  else group_gather_update<3><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff, store_a);
   if (g->n_rec > 0) {
     const int32_t *own_rec = own + g->n_stiff + g->n_gather;
     if (g->c == 1) group_receivers<1><<<(unsigned)g->n_rec, kRecThreads, 0, g->stream>>>(slots, own_rec, P);
@@ -2215,7 +2231,11 @@ int salvus_problem_destroy(salvus_problem *p) {
 int salvus_problem_set_dt(salvus_problem *p, double dt) {
   if (!p) return fail(SALVUS_E_INVALID, "null problem");
   if (!(dt > 0) || !std::isfinite(dt)) return fail(SALVUS_E_INVALID, "dt must be positive");
-  if (p->dt != dt) drop_graph(p);
+  if (p->dt != dt) {
+    drop_graph(p);
+    SALVUS_CUDA(cudaSetDevice(p->mesh->device));
+    if (int rc = velocity_form(p, false)) return rc;  // w belongs to the old step
+  }
   p->dt = dt;
   p->dt_set = true;
   return SALVUS_OK;
@@ -2522,6 +2542,11 @@ int salvus_problem_set_field(salvus_problem *p, int32_t f, int32_t shot, const d
   if (!b || shot != 0) return fail(SALVUS_E_INVALID, "bad field %d / shot %d", f, shot);
   const size_t N = (size_t)p->mesh->G * p->c;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
+  if (f == SALVUS_FIELD_V) {
+    p->half_step = false;  // v as given; w is formed before the next step
+  } else if (f == SALVUS_FIELD_A_PREV) {
+    if (int rc = velocity_form(p, false)) return rc;  // v does not change with a_
+  }
   if (p->prec == SALVUS_FP64) {
     int rc = copy_h2d(p, b->ptr, vals, 8 * N);
     if (rc) return rc;
@@ -2541,14 +2566,25 @@ int salvus_problem_get_field(salvus_problem *p, int32_t f, int32_t shot, double 
   if (!b || shot != 0) return fail(SALVUS_E_INVALID, "bad field %d / shot %d", f, shot);
   const size_t N = (size_t)p->mesh->G * p->c;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
-  if (p->prec == SALVUS_FP64) {
+  const bool from_w = f == SALVUS_FIELD_V && p->half_step;
+  if (p->prec == SALVUS_FP64 && !from_w) {
     int rc = copy_d2h(p, vals, b->ptr, 8 * N);
     if (rc) return rc;
   } else {
     int rc;
     if (p->d_stage.bytes < 8 * N && (rc = p->d_stage.alloc(8 * N))) return rc;
-    convert_kernel<float, double><<<blocks_for((int64_t)N, 256), 256, 0, p->stream>>>(
-        (int64_t)N, b->as<float>(), p->d_stage.as<double>());
+    const unsigned grid = blocks_for((int64_t)N, 256);
+    if (!from_w)
+      convert_kernel<float, double><<<grid, 256, 0, p->stream>>>((int64_t)N, b->as<float>(),
+                                                                 p->d_stage.as<double>());
+    else if (p->prec == SALVUS_FP32)
+      velocity_kernel<float><<<grid, 256, 0, p->stream>>>((int64_t)N, b->as<float>(),
+                                                          p->d_ap.as<float>(), (float)(0.5 * p->dt),
+                                                          p->d_stage.as<double>());
+    else
+      velocity_kernel<double><<<grid, 256, 0, p->stream>>>((int64_t)N, b->as<double>(),
+                                                           p->d_ap.as<double>(), 0.5 * p->dt,
+                                                           p->d_stage.as<double>());
     g_launches++;
     if ((rc = check_launch("convert"))) return rc;
     if ((rc = copy_d2h(p, vals, p->d_stage.ptr, 8 * N))) return rc;
@@ -2570,6 +2606,7 @@ int salvus_assemble(salvus_problem *p) {
   rc = ready(p);
   if (rc) return rc;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
+  if ((rc = velocity_form(p, true))) return rc;  // the coupling terms read v through w
   return by_components(p->c, [&](auto cc) {
     constexpr int C = decltype(cc)::value;
     return p->prec == SALVUS_FP32 ? assemble_t<float, C>(p) : assemble_t<double, C>(p);
@@ -2594,6 +2631,7 @@ int salvus_take_time_step(salvus_problem *p) {
   rc = ready(p);
   if (rc) return rc;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
+  if ((rc = velocity_form(p, true))) return rc;
   rc = by_components(p->c, [&](auto cc) {
     constexpr int C = decltype(cc)::value;
     return p->prec == SALVUS_FP32 ? newmark_t<float, C>(p) : newmark_t<double, C>(p);
@@ -2607,7 +2645,8 @@ int salvus_step(salvus_problem *p) {
   int rc = ready(p);
   if (rc) return rc;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
-  rc = step_fused(p);
+  if ((rc = velocity_form(p, true))) return rc;
+  rc = step_fused(p, true);
   if (rc == SALVUS_OK) p->step++;
   if (rc == SALVUS_OK && p->step % kFiniteEvery == 0) rc = launch_finite_check(p);
   return rc;
@@ -2657,7 +2696,7 @@ static int capture_steps(salvus_problem *p, int steps, cudaGraphExec_t *exec, in
   SALVUS_CUDA(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
   int crc = SALVUS_OK;
   const int64_t l0 = g_launches.load();
-  for (int s = 0; s < steps && crc == SALVUS_OK; ++s) crc = step_fused(p);
+  for (int s = 0; s < steps && crc == SALVUS_OK; ++s) crc = step_fused(p, s == steps - 1);
   if (crc == SALVUS_OK) crc = launch_finite_check(p);
   // the captured sequence ends joined (a forked stream must rejoin the
   // capture), so every replay is self-contained
@@ -2716,6 +2755,7 @@ int salvus_run(salvus_problem *p, int64_t n_steps, int32_t mode) {
     return fail(SALVUS_E_INVALID, "unknown run mode %d", mode);
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
   if ((rc = rec_stream_ready(p))) return rc;
+  if (n_steps > 0 && (rc = velocity_form(p, true))) return rc;
   return run_steps(p, n_steps, mode);
 }
 
@@ -2731,7 +2771,7 @@ int salvus_problem_prepare_run(salvus_problem *p, int64_t n_steps) {
 static int plain_steps(salvus_problem *p, int64_t n) {
   int rc;
   for (int64_t s = 0; s < n; ++s) {
-    if ((rc = step_fused(p))) return rc;
+    if ((rc = step_fused(p, s == n - 1))) return rc;
     p->step++;
     if (p->step % kFiniteEvery == 0 && (rc = launch_finite_check(p))) return rc;
   }
@@ -2783,7 +2823,8 @@ static int energy_t(salvus_problem *p, double *kinetic, double *strain) {
   g_launches++;
   if ((rc = check_launch("energy gather"))) return rc;
   energy_kernel<real, C><<<kBlocks, 256, 0, p->stream>>>(
-      m->G, F<real>(p->d_u), F<real>(p->d_v), p->d_escr.as<real>(), m->d_mi64.as<double>(),
+      m->G, F<real>(p->d_u), F<real>(p->d_v), F<real>(p->d_ap),
+      p->half_step ? (real)(0.5 * p->dt) : real(0), p->d_escr.as<real>(), m->d_mi64.as<double>(),
       p->d_epart.as<double>());
   g_launches++;
   if ((rc = check_launch("energy"))) return rc;
@@ -2991,6 +3032,8 @@ int salvus_group_run(salvus_group *g, int64_t n_steps) {
   if (!g) return fail(SALVUS_E_INVALID, "null group");
   if (n_steps < 0) return fail(SALVUS_E_INVALID, "negative step count");
   SALVUS_CUDA(cudaSetDevice(g->m0->device));
+  for (auto *p : g->members)
+    if (int rc = velocity_form(p, true)) return rc;
   // order the group after every member's pending work
   for (size_t k = 0; k < g->members.size(); ++k) {
     SALVUS_CUDA(cudaEventRecord(g->member_ev[k], g->members[k]->stream));
@@ -3008,7 +3051,7 @@ int salvus_group_run(salvus_group *g, int64_t n_steps) {
     cudaGraph_t graph;
     SALVUS_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
     int crc = SALVUS_OK;
-    for (int s = 0; s < chunk && crc == SALVUS_OK; ++s) crc = group_step(g);
+    for (int s = 0; s < chunk && crc == SALVUS_OK; ++s) crc = group_step(g, s == chunk - 1);
     cudaError_t ce = cudaStreamEndCapture(g->stream, &graph);
     if (crc) return crc;
     if (ce != cudaSuccess) return fail(SALVUS_E_CUDA, "graph capture failed: %s", cudaGetErrorString(ce));
@@ -3025,7 +3068,7 @@ int salvus_group_run(salvus_group *g, int64_t n_steps) {
     done += g->graph_steps;
   }
   for (; done < n_steps; ++done)
-    if ((rc = group_step(g))) return rc;
+    if ((rc = group_step(g, done == n_steps - 1))) return rc;
   for (auto *p : g->members) p->step += n_steps;
   // members' later work waits for the group; then each member's finite check
   // on its own stream

@@ -162,6 +162,10 @@ struct salvus_problem {
   bool dt_set = false;
   int64_t step = 0;
   size_t rsize = 4;  // sizeof(real)
+  // what d_v holds: the reference's v (a field a caller has set, or the start
+  // at rest, where both are zero), or the half-step velocity w = v + dt/2 a_
+  // that the steps advance (newmark_point); velocity_form converts
+  bool half_step = false;
   salvus::DeviceBuffer d_u, d_v, d_a, d_ap, d_r;
   salvus::DeviceBuffer d_step;   // int64 device step counter
   salvus::DeviceBuffer d_stage;  // FP64 staging for host field copies

@@ -32,7 +32,7 @@ struct GroupSlot {
   const float *mi;
   int64_t E, G;
   // problem
-  float *u, *v, *ap, *a, *r;
+  float *u, *w, *ap, *r;  // w: half-step velocity
   float dt;
   double dtd;
   int64_t *step;
@@ -90,10 +90,11 @@ __global__ void group_source(const GroupSlot *__restrict__ slots, int P) {
 
 template <int C>
 __global__ void group_gather_update(const GroupSlot *__restrict__ slots,
-                                    const int32_t *__restrict__ owner) {
+                                    const int32_t *__restrict__ owner, bool store_a) {
   const GroupSlot &m = slots[owner[blockIdx.x]];
   const int64_t g = (blockIdx.x - m.b_gather) * (int64_t)blockDim.x + threadIdx.x;
-  gather_body<float, C, 0>(g, m.G, m.inc_off, m.inc_idx, m.r, m.mi, m.u, m.v, m.ap, m.a, m.dt);
+  gather_body<float, C, 0>(g, m.G, m.inc_off, m.inc_idx, m.r, m.mi, m.u, m.w,
+                           store_a ? m.ap : nullptr, nullptr, m.dt);
 }
 
 template <int C>
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(128)
 group_persistent_step(const GroupSlot *__restrict__ slots, const GroupCounts *__restrict__ counts,
                       int J, const GroupWork *__restrict__ work, int64_t total,
                       int32_t *__restrict__ done /* [J][4] */, GroupSync *__restrict__ sync,
-                      DMatrix<float> Dm, int P, long long wait_limit) {
+                      DMatrix<float> Dm, int P, long long wait_limit, bool store_a) {
   constexpr int n2 = (N + 1) * (N + 1);
   constexpr int EPB = kHex ? (128 / n2 > 0 ? 128 / n2 : 1) : 1;
   __shared__ long long s_item;
@@ -200,7 +201,7 @@ group_persistent_step(const GroupSlot *__restrict__ slots, const GroupCounts *__
       case GI_GATHER:
         for (int b = w.first; b < w.first + w.count; ++b)
           gather_body<float, C, 0, true>((int64_t)b * blockDim.x + t, m.G, m.inc_off, m.inc_idx, m.r, m.mi,
-                                   m.u, m.v, m.ap, m.a, m.dt);
+                                   m.u, m.w, store_a ? m.ap : nullptr, nullptr, m.dt);
         break;
       case GI_REC:
         receiver_body<float, C, true>(w.first, P, m.rec_elem, m.rec_l, m.conn, m.u, m.seis, m.cap, m.step);
@@ -257,7 +258,7 @@ template <int N, bool kHex, int C>
 __global__ void __launch_bounds__(128, kHex ? 5 : 10)
 group_partitioned_step(const GroupSlot *__restrict__ slots, const GroupPart *__restrict__ parts,
                        int J, GroupBar *__restrict__ bars, GroupSync *__restrict__ sync,
-                       DMatrix<float> Dm, int P, long long wait_limit) {
+                       DMatrix<float> Dm, int P, long long wait_limit, bool store_a) {
   constexpr int n2 = (N + 1) * (N + 1);
   constexpr int EPB = kHex ? (128 / n2 > 0 ? 128 / n2 : 1) : 1;
   __shared__ int s_ok;
@@ -310,7 +311,7 @@ group_partitioned_step(const GroupSlot *__restrict__ slots, const GroupPart *__r
   if (ok)
     for (int k = b; k < pt.n_gather; k += nb)
       gather_body<float, C, 0, true>((int64_t)k * 128 + t, m.G, m.inc_off, m.inc_idx, m.r, m.mi,
-                                     m.u, m.v, m.ap, m.a, m.dt);
+                                     m.u, m.w, store_a ? m.ap : nullptr, nullptr, m.dt);
   arrive(&gb->gather_done);
   ok = ok && member_wait(&gb->gather_done, nb);
   // receivers

@@ -40,7 +40,7 @@ namespace salvus {
 // source kernel after the source terms are added: source_interior_body).
 struct HexInteriorUpdate {
   const float *mi;
-  float *v, *ap;
+  float *w, *ap;  // ap: null unless this step stores a_
   float dt;
   int nsrc_elem;
   const int64_t *src_elem;  // distinct source elements
@@ -163,7 +163,7 @@ __device__ __forceinline__ void elastic_hex_affine_body(
   const bool icol = kFuse && i >= 1 && i <= n - 2 && j >= 1 && j <= n - 2;
   // Elements holding a source keep the unfused form for their interior
   // points (residuals written; the source kernel adds the source terms and
-  // finishes those nodes).  For the others, the interior operands (v, a_)
+  // finishes those nodes).  For the others, the interior operands (w)
   // are loaded here, before the divergence, so that their latency overlaps
   // it (after the stores below the compiler could not reorder them: the
   // pointers may alias as far as it knows).
@@ -171,19 +171,15 @@ __device__ __forceinline__ void elastic_hex_affine_body(
   if constexpr (kFuse) {
     for (int s = 0; s < iu.nsrc_elem && fuse_here; ++s) fuse_here = __ldg(iu.src_elem + s) != e;
   }
-  float vpre[n][3], apre[n][3];
+  float wpre[n][3];
   if constexpr (kFuse) {
     if (fuse_here) {
-      const float *__restrict__ vv = iu.v;
-      const float *__restrict__ aa = iu.ap;
+      const float *__restrict__ ww = iu.w;
 #pragma unroll
       for (int k = 1; k < n - 1; ++k) {
         const int64_t g = node[k];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          vpre[k][c] = vv[g * 3 + c];
-          apre[k][c] = aa[g * 3 + c];
-        }
+        for (int c = 0; c < 3; ++c) wpre[k][c] = ww[g * 3 + c];
       }
     }
   }
@@ -218,12 +214,12 @@ __device__ __forceinline__ void elastic_hex_affine_body(
       for (int c = 0; c < 3; ++c) {
         const int64_t x = g * 3 + c;
         float uo = c == 0 ? ux[k] : (c == 1 ? uy[k] : uz[k]);
-        float vo = vpre[k][c], apo = apre[k][c];
-        const float acc = add_rn(0.f, o[c]);
-        newmark_point<float>(mul_rn(acc, mm), apo, vo, uo, iu.dt);
+        float wo = wpre[k][c];
+        const float an = mul_rn(add_rn(0.f, o[c]), mm);
+        newmark_point<float>(an, wo, uo, iu.dt);
         u[x] = uo;
-        iu.v[x] = vo;
-        iu.ap[x] = apo;
+        iu.w[x] = wo;
+        if (iu.ap) iu.ap[x] = an;
       }
     }
   }
@@ -244,7 +240,7 @@ __global__ void source_fused_hex_kernel(int nsrc, int P, const int64_t *__restri
                                        const int64_t *__restrict__ src_elems,
                                        const int32_t *__restrict__ conn,
                                        const float *__restrict__ mi, float *__restrict__ u,
-                                       float *__restrict__ v, float *__restrict__ ap, float dt) {
+                                       float *__restrict__ w, float *__restrict__ ap, float dt) {
   source_body<float, 3>(nsrc, P, elem, par, wts, step, dtd, r);  // ends with __syncthreads
   constexpr int n = N + 1, m = N - 1, NI = m * m * m;
   for (int t = threadIdx.x; t < nse * NI * 3; t += blockDim.x) {
@@ -253,11 +249,12 @@ __global__ void source_fused_hex_kernel(int nsrc, int P, const int64_t *__restri
     const int64_t e = src_elems[se];
     const int pt = i + n * j + n * n * k;
     const int64_t g = conn[e * P + pt], x = g * 3 + c;
-    float uo = u[x], vo = v[x], apo = ap[x];
-    newmark_point<float>(mul_rn(add_rn(0.f, r[(e * P + pt) * 3 + c]), mi[g]), apo, vo, uo, dt);
+    float uo = u[x], wo = w[x];
+    const float an = mul_rn(add_rn(0.f, r[(e * P + pt) * 3 + c]), mi[g]);
+    newmark_point<float>(an, wo, uo, dt);
     u[x] = uo;
-    v[x] = vo;
-    ap[x] = apo;
+    w[x] = wo;
+    if (ap) ap[x] = an;
   }
 }
 

@@ -8,7 +8,8 @@
 //                   points in ascending element order (deterministic);
 //   inverse mass    Order2Newmark::applyInverseMassMatrix (Order2Newmark.cpp:68-83);
 //   Newmark         Order2Newmark::takeTimeStep (Order2Newmark.cpp:85-114):
-//                   v += dt/2 (a + a_), u += dt v + dt^2/2 a, a_ = a;
+//                   v += dt/2 (a + a_), u += dt v + dt^2/2 a, a_ = a, kept in
+//                   the half-step velocity w = v + dt/2 a_ (newmark_point);
 //   source          Scalar::computeSourceTerm (Scalar.cpp:79-88),
 //                   Elastic3D::computeSourceTerm (Elastic3D.cpp:126-133),
 //                   Ricker::fire (Ricker.cpp:27-33), evaluated at t_n = n dt;
@@ -21,7 +22,7 @@
 
 namespace salvus {
 
-// One Newmark update with explicitly rounded operations, so that the fused
+// Explicitly rounded operations for the update, so that the fused
 // gather/update kernel and the three-call path (gather, inverse mass,
 // Newmark) produce bitwise identical wavefields whatever the compiler's
 // contraction choices.
@@ -29,18 +30,46 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// One Newmark update on the half-step velocity w = v + dt/2 a_.  The
+// reference's v += dt/2 (a + a_), u += dt v + dt^2/2 a, a_ = a
+// (Order2Newmark.cpp:104-108) is, with w, the two operations below: v after
+// the step is w - dt/2 a with the step's a, which is needed only when a
+// caller asks for v (half_step_velocity).  A step therefore reads and writes
+// u and w alone: 4 field streams instead of 6 (u, v and a_ both ways), which
+// is what bounds the node gather (DRAM).  On 17 M nodes x 3 components that
+// is 48 instead of 72 bytes per node: 32 steps of the 64^3 order-4 elastic
+// mesh took 26.7 ms before and take 23.9 ms (B200).
 template <typename real>
-__device__ __forceinline__ void newmark_point(real an, real &ap, real &v, real &u, real dt) {
-  const real acl = mul_rn(real(0.5), dt), dsp = mul_rn(mul_rn(real(0.5), dt), dt);
-  // v_{n} = dt/2 a + dt/2 a_ + v ; u = dt v + dt^2/2 a + u  (Order2Newmark.cpp:104-107)
-  const real vn = add_rn(add_rn(mul_rn(acl, an), mul_rn(acl, ap)), v);
-  u = add_rn(add_rn(mul_rn(dt, vn), mul_rn(dsp, an)), u);
-  v = vn;
-  ap = an;
+__device__ __forceinline__ void newmark_point(real an, real &w, real &u, real dt) {
+  w = fma_rn(dt, an, w);
+  u = fma_rn(dt, w, u);
 }
 
-// mode 0: fused  a = mi * sum(r); Newmark update of (u, v, a_)
+// The velocity at a whole step from the stored pair (hdt = dt/2), and back.
+template <typename real>
+__device__ __forceinline__ real half_step_velocity(real w, real ap, real hdt) {
+  return fma_rn(-hdt, ap, w);
+}
+// x <- x + s y: v -> w (s = dt/2) and w -> v (s = -dt/2) in place.
+template <typename real>
+__global__ void axpy_kernel(int64_t N, real s, const real *__restrict__ y, real *__restrict__ x) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < N) x[i] = fma_rn(s, y[i], x[i]);
+}
+// out = w - dt/2 a_ in FP64, the velocity field a caller reads.
+template <typename real>
+__global__ void velocity_kernel(int64_t N, const real *__restrict__ w, const real *__restrict__ ap,
+                                real hdt, double *__restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < N) out[i] = (double)half_step_velocity<real>(w[i], ap[i], hdt);
+}
+
+// mode 0: fused  a = mi * sum(r); Newmark update of (u, w); a_ = a is stored
+//         when ap is not null (the last step of a run: later steps never read
+//         it, only callers do)
 // mode 1: gather a = sum(r)
 // kInKernelR: r was written earlier in the same launch (fused group steps)
 // and is read with coherent loads (ld.global.ca), not ld.global.nc.
@@ -49,19 +78,18 @@ __device__ __forceinline__ void gather_body(int64_t g, int64_t G, const int32_t 
                                             const int32_t *__restrict__ idx,
                                             const real *__restrict__ r,
                                             const real *__restrict__ mi, real *__restrict__ u,
-                                            real *__restrict__ v, real *__restrict__ ap,
+                                            real *__restrict__ w, real *__restrict__ ap,
                                             real *__restrict__ a, real dt) {
   if (g >= G) return;
   // Newmark operands first: they do not depend on the gather, so their loads
   // overlap the dependent index -> residual chain below.
-  real m = 0, uo[C], vo[C], apo[C];
+  real m = 0, uo[C], wo[C];
   if (MODE == 0) {
     m = mi[g];
 #pragma unroll
     for (int c = 0; c < C; ++c) {
       uo[c] = u[g * C + c];
-      vo[c] = v[g * C + c];
-      apo[c] = ap[g * C + c];
+      wo[c] = w[g * C + c];
     }
   }
   real acc[C];
@@ -122,10 +150,11 @@ __device__ __forceinline__ void gather_body(int64_t g, int64_t G, const int32_t 
 #pragma unroll
     for (int c = 0; c < C; ++c) {
       const int64_t i = g * C + c;
-      newmark_point<real>(mul_rn(acc[c], m), apo[c], vo[c], uo[c], dt);
+      const real an = mul_rn(acc[c], m);
+      newmark_point<real>(an, wo[c], uo[c], dt);
       u[i] = uo[c];
-      v[i] = vo[c];
-      ap[i] = apo[c];
+      w[i] = wo[c];
+      if (ap) ap[i] = an;
     }
   }
 }
@@ -134,10 +163,10 @@ template <typename real, int C, int MODE>
 __global__ void gather_kernel(int64_t G, const int32_t *__restrict__ off,
                               const int32_t *__restrict__ idx, const real *__restrict__ r,
                               const real *__restrict__ mi, real *__restrict__ u,
-                              real *__restrict__ v, real *__restrict__ ap, real *__restrict__ a,
+                              real *__restrict__ w, real *__restrict__ ap, real *__restrict__ a,
                               real dt) {
   gather_body<real, C, MODE>((int64_t)blockIdx.x * blockDim.x + threadIdx.x, G, off, idx, r, mi, u,
-                             v, ap, a, dt);
+                             w, ap, a, dt);
 }
 
 // The gather / update over a list of nodes (the shared nodes of a fused
@@ -147,11 +176,11 @@ __global__ void gather_list_kernel(int64_t n, const int32_t *__restrict__ nodes,
                                    const int32_t *__restrict__ off,
                                    const int32_t *__restrict__ idx, const real *__restrict__ r,
                                    const real *__restrict__ mi, real *__restrict__ u,
-                                   real *__restrict__ v, real *__restrict__ ap,
+                                   real *__restrict__ w, real *__restrict__ ap,
                                    real *__restrict__ a, real dt) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  gather_body<real, C, MODE>(nodes[t], INT64_MAX, off, idx, r, mi, u, v, ap, a, dt);
+  gather_body<real, C, MODE>(nodes[t], INT64_MAX, off, idx, r, mi, u, w, ap, a, dt);
 }
 
 // Blow-up detection: any NaN / Inf among n values sets the problem's device
@@ -186,19 +215,21 @@ __global__ void dirichlet_zero_kernel(int64_t n, const int32_t *__restrict__ pts
 // summed over the element's coupled edges; the first n_fluid points belong to
 // fluid elements (u += cx vx + cy vy), the rest to solid elements
 // (ux += cx v, uy += cy v).  Runs after the stiffness (and Dirichlet zeroing)
-// and before the sources, on the velocity field.
+// and before the sources, on the velocity field v = w - dt/2 a_ (these meshes
+// store a_ at every step for it).
 template <typename real>
 __global__ void coupling_kernel(int64_t n_fluid, int64_t n, const int32_t *__restrict__ pts,
-                                const real *__restrict__ coef, const real *__restrict__ v,
-                                real *__restrict__ r) {
+                                const real *__restrict__ coef, const real *__restrict__ w,
+                                const real *__restrict__ ap, real hdt, real *__restrict__ r) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t ep = pts[2 * i], g = pts[2 * i + 1];
   const real cx = coef[2 * i], cy = coef[2 * i + 1];
+  auto v = [&](int64_t x) { return half_step_velocity<real>(w[x], ap[x], hdt); };
   if (i < n_fluid) {
-    r[ep * 3] += cx * v[g * 3 + 1] + cy * v[g * 3 + 2];
+    r[ep * 3] += cx * v(g * 3 + 1) + cy * v(g * 3 + 2);
   } else {
-    const real vf = v[g * 3];
+    const real vf = v(g * 3);
     r[ep * 3 + 1] += cx * vf;
     r[ep * 3 + 2] += cy * vf;
   }
@@ -213,14 +244,15 @@ __global__ void inverse_mass_kernel(int64_t G, const real *__restrict__ mi, real
 
 template <typename real>
 __global__ void newmark_kernel(int64_t N, const real *__restrict__ a, real *__restrict__ u,
-                               real *__restrict__ v, real *__restrict__ ap, real dt) {
+                               real *__restrict__ w, real *__restrict__ ap, real dt) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  real apv = ap[i], vv = v[i], uv = u[i];
-  newmark_point<real>(a[i], apv, vv, uv, dt);
+  const real an = a[i];
+  real wv = w[i], uv = u[i];
+  newmark_point<real>(an, wv, uv, dt);
   u[i] = uv;
-  v[i] = vv;
-  ap[i] = apv;
+  w[i] = wv;
+  ap[i] = an;
 }
 
 __device__ __forceinline__ double ricker_dev(double t, double f0, double t0, double amp) {
@@ -341,13 +373,13 @@ __global__ void dot_kernel(int64_t N, int C, const real *__restrict__ x, const r
 // compensation, the CTA adds the threads' sums in a fixed tree order, and
 // partial[2 * block] / [2 * block + 1] (kinetic, strain) are summed on the
 // host in block order -- the same bits on every run for a given grid.
-// ku = -K u (the gathered stiffness action); M = 1 / mi per node, nodes
-// without mass (mi = 0) carry none.
+// ku = -K u (the gathered stiffness action); v = w - dt/2 a_; M = 1 / mi per
+// node, nodes without mass (mi = 0) carry none; hdt = 0: w holds v itself.
 template <typename real, int C>
 __global__ void __launch_bounds__(256)
-energy_kernel(int64_t G, const real *__restrict__ u, const real *__restrict__ v,
-              const real *__restrict__ ku, const double *__restrict__ mi,
-              double *__restrict__ partial) {
+energy_kernel(int64_t G, const real *__restrict__ u, const real *__restrict__ w,
+              const real *__restrict__ ap, real hdt, const real *__restrict__ ku,
+              const double *__restrict__ mi, double *__restrict__ partial) {
   __shared__ double sk[256], ss[256];
   double ek = 0.0, ck = 0.0, es = 0.0, cs = 0.0;
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < G;
@@ -355,7 +387,9 @@ energy_kernel(int64_t G, const real *__restrict__ u, const real *__restrict__ v,
     const double m = mi[g] != 0.0 ? 1.0 / mi[g] : 0.0;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-      const double vv = (double)v[g * C + c], uu = (double)u[g * C + c];
+      const real wv = w[g * C + c];
+      const double vv = hdt != 0 ? (double)half_step_velocity<real>(wv, ap[g * C + c], hdt) : (double)wv;
+      const double uu = (double)u[g * C + c];
       const double yk = 0.5 * m * vv * vv - ck;
       const double tk = ek + yk;
       ck = (tk - ek) - yk;
