@@ -1,7 +1,7 @@
 // abi.cu -- extern "C" entry points (include/salvus_b200.h): mesh flattening,
 // device residency, and the per-step launch sequence
-//   stiffness (element-local residual) -> sources -> node gather + inverse
-//   mass + Newmark -> receivers.
+//   stiffness (element-local residual) -> node gather with the sources +
+//   inverse mass + Newmark -> receivers.
 #include <cuda_runtime.h>
 
 #include <unistd.h>
@@ -667,21 +667,66 @@ static int mesh_setup_device(salvus_mesh *m) {
 template <typename real>
 static real *F(const DeviceBuffer &b) { return b.as<real>(); }
 
+// The node gather's view of the sources (SourceTerms).  el: the sources'
+// elements, ascending (an element's sources adjacent).
+static void source_tiles(const salvus_mesh *m, const std::vector<int64_t> &el,
+                         std::vector<int32_t> &tile, std::vector<int4> &node) {
+  const int4 none{0, 0, 0, -1};
+  tile.assign((size_t)((m->G + kSrcTile - 1) / kSrcTile), -1);
+  size_t tiles = 0;
+  for (size_t s = 0; s < el.size(); ++s)
+    for (int q = 0; q < m->P; ++q) {
+      int32_t &t = tile[(size_t)(m->conn[(size_t)(el[s] * m->P + q)] / kSrcTile)];
+      if (t < 0) t = (int32_t)(kSrcTile * tiles++);
+    }
+  node.assign(kSrcTile * tiles, none);
+  for (size_t s = 0; s < el.size();) {
+    size_t t = s;
+    while (t < el.size() && el[t] == el[s]) ++t;
+    for (int q = 0; q < m->P; ++q) {
+      const int32_t g = m->conn[(size_t)(el[s] * m->P + q)];
+      size_t at = (size_t)(tile[(size_t)(g / kSrcTile)] + g % kSrcTile);
+      if (node[at].z > 0) {  // a node of another source element too: append
+        while (node[at].w >= 0) at = (size_t)node[at].w;
+        node[at].w = (int32_t)node.size();
+        at = node.size();
+        node.push_back(none);
+      }
+      node[at] = int4{(int32_t)(s * m->P + q), (int32_t)s, (int32_t)(t - s), -1};
+    }
+    s = t;
+  }
+}
+
+static SourceTerms source_terms(const salvus_problem *p) {
+  SourceTerms s;
+  if (p->srcs.empty()) return s;
+  s.tile = p->src_tile;
+  s.node = p->src_node;
+  s.wts = p->src_wts;
+  s.stf = p->stf;
+  s.P = p->mesh->P;
+  return s;
+}
+
 static int upload_sources(salvus_problem *p) {
   if (!p->src_dirty) return SALVUS_OK;
   const salvus_mesh *m = p->mesh;
   const size_t ns = p->srcs.size();
-  int rc;
+  p->n_src_uelem = 0;
   if (ns) {
-    // batched problems group sources by shot (attach order kept within a shot)
+    // batched problems group sources by shot, single-shot ones by element
+    // (attach order kept within each)
     std::vector<size_t> order(ns);
     for (size_t s = 0; s < ns; ++s) order[s] = s;
     std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
-      return p->srcs[a].desc.shot < p->srcs[b].desc.shot;
+      return p->shots > 1 ? p->srcs[a].desc.shot < p->srcs[b].desc.shot
+                          : p->srcs[a].elem < p->srcs[b].elem;
     });
-    std::vector<int64_t> el(ns);
+    std::vector<int64_t> el(ns), ue;
     std::vector<double> par(3 * ns), w(ns * m->P * p->c);
-    std::vector<int32_t> shot_off(p->shots_pad + 1, 0);
+    std::vector<int32_t> shot_off(p->shots_pad + 1, 0), tile;
+    std::vector<int4> node;
     for (size_t k = 0; k < ns; ++k) {
       const auto &src = p->srcs[order[k]];
       el[k] = src.elem;
@@ -690,33 +735,44 @@ static int upload_sources(salvus_problem *p) {
       par[3 * k + 2] = src.desc.amplitude;
       std::memcpy(&w[k * m->P * p->c], src.wts.data(), sizeof(double) * m->P * p->c);
       shot_off[src.desc.shot + 1]++;
+      // distinct source elements (fused hexahedron step)
+      if (p->shots == 1 && (ue.empty() || ue.back() != src.elem)) ue.push_back(src.elem);
     }
     for (int s = 0; s < p->shots_pad; ++s) shot_off[s + 1] += shot_off[s];
-    if ((rc = p->d_shot_off.alloc(sizeof(int32_t) * shot_off.size()))) return rc;
-    SALVUS_CUDA(cudaMemcpyAsync(p->d_shot_off.ptr, shot_off.data(), sizeof(int32_t) * shot_off.size(),
-                                cudaMemcpyHostToDevice, p->stream));
-    if ((rc = p->d_src_elem.alloc(sizeof(int64_t) * ns))) return rc;
-    if ((rc = p->d_src_par.alloc(sizeof(double) * par.size()))) return rc;
-    if ((rc = p->d_src_wts.alloc(sizeof(double) * w.size()))) return rc;
-    SALVUS_CUDA(cudaMemcpyAsync(p->d_src_elem.ptr, el.data(), sizeof(int64_t) * ns,
-                                cudaMemcpyHostToDevice, p->stream));
-    SALVUS_CUDA(cudaMemcpyAsync(p->d_src_par.ptr, par.data(), sizeof(double) * par.size(),
-                                cudaMemcpyHostToDevice, p->stream));
-    SALVUS_CUDA(cudaMemcpyAsync(p->d_src_wts.ptr, w.data(), sizeof(double) * w.size(),
-                                cudaMemcpyHostToDevice, p->stream));
-    // distinct source elements, first appearance order (fused hexahedron step)
-    std::vector<int64_t> ue;
-    for (int64_t x : el)
-      if (std::find(ue.begin(), ue.end(), x) == ue.end()) ue.push_back(x);
-    if ((rc = p->d_src_uelem.alloc(sizeof(int64_t) * ue.size()))) return rc;
-    SALVUS_CUDA(cudaMemcpyAsync(p->d_src_uelem.ptr, ue.data(), sizeof(int64_t) * ue.size(),
-                                cudaMemcpyHostToDevice, p->stream));
+    if (p->shots == 1) source_tiles(m, el, tile, node);
+    // one host image, one allocation and one copy
+    std::vector<char> img;
+    auto put = [&](const void *data, size_t bytes) {
+      const size_t at = (img.size() + 15) & ~size_t(15);
+      img.resize(at + bytes);
+      if (data) std::memcpy(img.data() + at, data, bytes);
+      return at;
+    };
+    const size_t o_el = put(el.data(), sizeof(int64_t) * ns);
+    const size_t o_ue = put(ue.data(), sizeof(int64_t) * ue.size());
+    const size_t o_par = put(par.data(), sizeof(double) * par.size());
+    const size_t o_w = put(w.data(), sizeof(double) * w.size());
+    const size_t o_so = put(shot_off.data(), sizeof(int32_t) * shot_off.size());
+    const size_t o_t = put(tile.data(), sizeof(int32_t) * tile.size());
+    const size_t o_n = put(node.data(), sizeof(int4) * node.size());
+    const size_t o_stf = put(nullptr, sizeof(double) * ns);
+    int rc = p->d_src.alloc(img.size());
+    if (rc) return rc;
+    char *d = p->d_src.as<char>();
+    p->src_elem = (const int64_t *)(d + o_el);
+    p->src_uelem = (const int64_t *)(d + o_ue);
+    p->src_par = (const double *)(d + o_par);
+    p->src_wts = (const double *)(d + o_w);
+    p->shot_off = (const int32_t *)(d + o_so);
+    p->src_tile = (const int32_t *)(d + o_t);
+    p->src_node = (const int4 *)(d + o_n);
+    p->stf = (double *)(d + o_stf);
     p->n_src_uelem = (int)ue.size();
+    SALVUS_CUDA(cudaMemcpyAsync(d, img.data(), img.size(), cudaMemcpyHostToDevice, p->stream));
     SALVUS_CUDA(cudaStreamSynchronize(p->stream));
-  } else {
-    p->n_src_uelem = 0;
   }
   p->src_dirty = false;
+  p->stf_ready = false;
   return SALVUS_OK;
 }
 
@@ -776,25 +832,15 @@ static int launch_dirichlet(salvus_problem *p) {
   return check_launch("dirichlet");
 }
 
-template <typename real, int C>
-static int launch_sources(salvus_problem *p) {
-  if (p->srcs.empty()) return SALVUS_OK;
-  ProfScope ps(p, K_SRC);
-  source_kernel<real, C><<<1, 256, 0, p->stream>>>(
-      (int)p->srcs.size(), p->mesh->P, p->d_src_elem.as<int64_t>(), p->d_src_par.as<double>(),
-      p->d_src_wts.as<double>(), p->d_step.as<int64_t>(), p->dt, F<real>(p->d_r));
-  g_launches++;
-  return check_launch("source");
-}
-
-// Receivers of step n read u after its update and advance the device step
-// counter; step n + 1's stiffness launch only reads u.  In the steps a
-// graph run captures (rec_overlap) they therefore run on a second stream,
-// forked after the node update, and step n + 1 joins them after its
-// stiffness launch, before its sources (which read the step counter) and
-// its node update (which writes u); the captured sequence ends joined, so
-// every later operation on the problem's stream is ordered after them.
-// Host-launched and profiled steps keep them on the problem's stream.
+// The tail of step n (step_tail_kernel) samples its receivers, which read u
+// after its update, and evaluates the sources of step n + 1, whose stiffness
+// launch only reads u.  In the steps a graph run captures (rec_overlap) it
+// therefore runs on a second stream, forked after the node update, and step
+// n + 1 joins it after its stiffness launch, before its node update (which
+// writes u and advances the step counter): off the critical path, which is
+// two launches.  The captured sequence ends joined, so every later operation
+// on the problem's stream is ordered after it.  Host-launched and profiled
+// steps keep it on the problem's stream.
 static int join_receivers(salvus_problem *p) {
   if (!p->rec_pending) return SALVUS_OK;
   p->rec_pending = false;
@@ -803,30 +849,41 @@ static int join_receivers(salvus_problem *p) {
 }
 
 template <typename real, int C>
+static int launch_step_tail(salvus_problem *p, int nrec, cudaStream_t st) {
+  const int nsrc = (int)p->srcs.size(), blocks = nrec + (nsrc > 0 ? 1 : 0);
+  if (blocks == 0) return SALVUS_OK;
+  step_tail_kernel<real, C><<<blocks, kRecThreads, 0, st>>>(
+      nrec, p->mesh->P, p->d_rec_elem.as<int64_t>(), p->d_rec_l.as<double>(),
+      p->mesh->d_conn.as<int32_t>(), F<real>(p->d_u), p->d_seis.as<double>(), p->seis_cap,
+      p->d_step.as<int64_t>(), nsrc, p->src_par, p->dt, p->stf);
+  g_launches++;
+  return check_launch("receivers");
+}
+
+template <typename real, int C>
 static int launch_receivers(salvus_problem *p) {
   ProfScope ps(p, K_REC);
-  cudaStream_t st = p->stream;
+  const int nrec = (int)p->recs.size();
+  if (nrec == 0 && p->srcs.empty()) return SALVUS_OK;
   const bool fork = p->rec_overlap && !p->profiling && p->rec_stream;
-  if (fork) {
-    SALVUS_CUDA(cudaEventRecord(p->ev_updated, p->stream));
-    SALVUS_CUDA(cudaStreamWaitEvent(p->rec_stream, p->ev_updated, 0));
-    st = p->rec_stream;
-  }
-  const int nr = (int)p->recs.size();
-  if (nr > 0) {
-    receiver_kernel<real, C><<<nr, kRecThreads, 0, st>>>(
-        p->mesh->P, p->d_rec_elem.as<int64_t>(), p->d_rec_l.as<double>(),
-        p->mesh->d_conn.as<int32_t>(), F<real>(p->d_u), p->d_seis.as<double>(), p->seis_cap,
-        p->d_step.as<int64_t>());
-    g_launches++;
-  }
-  advance_step_kernel<<<1, 1, 0, st>>>(p->d_step.as<int64_t>());
-  g_launches++;
-  if (fork) {
-    SALVUS_CUDA(cudaEventRecord(p->ev_recorded, p->rec_stream));
-    p->rec_pending = true;
-  }
-  return check_launch("receivers");
+  if (!fork) return launch_step_tail<real, C>(p, nrec, p->stream);
+  SALVUS_CUDA(cudaEventRecord(p->ev_updated, p->stream));
+  SALVUS_CUDA(cudaStreamWaitEvent(p->rec_stream, p->ev_updated, 0));
+  int rc = launch_step_tail<real, C>(p, nrec, p->rec_stream);
+  SALVUS_CUDA(cudaEventRecord(p->ev_recorded, p->rec_stream));
+  p->rec_pending = true;
+  return rc;
+}
+
+// The source-time functions of the step that the device counter stands at,
+// where no tail has evaluated them (new sources, a new time step, steps of a
+// single-launch group).  Never inside a graph capture: the entry points call
+// it before they step or capture.
+static int sources_ready(salvus_problem *p) {
+  if (p->stf_ready || p->srcs.empty() || p->shots > 1) return SALVUS_OK;
+  ProfScope ps(p, K_SRC);
+  p->stf_ready = true;
+  return launch_step_tail<float, 1>(p, 0, p->stream);  // no receiver: the type does not matter
 }
 
 template <typename real>
@@ -842,9 +899,9 @@ static const real *inv_mass(const salvus_problem *p) {
 // element-interior nodes inside the stiffness kernel and gathers the rest
 // (kernels_hex_affine.cuh).  Measured on the 64^3 order-4 workload it is
 // slower than the plain sequence on the same records (the interior update
-// costs the stiffness kernel more than the shorter gather saves), so the
-// hexahedron autotuner (tune_hex) picks between the two per problem;
-// SALVUS_HEX_STEP=fused / plain forces the form (read at every step).  It is
+// costs the stiffness kernel more than the shorter gather saves, figures at
+// tune_hex), so it runs only where SALVUS_HEX_STEP=fused (read at every step)
+// or SALVUS_HEX_CONFIG asks for it.  It is
 // admissible for problems without Dirichlet points and with at most
 // kFuseMaxSources sources (each interior column scans their elements).
 constexpr int kFuseMaxSources = 16;
@@ -860,6 +917,10 @@ static bool hex_interior_fusion(const salvus_problem *p) {
   if (s && std::strcmp(s, "plain") == 0) return false;
   return p->hex_form == 1;
 }
+
+// 128-thread CTAs of the step's node gather: measured against 64 / 256 / 512
+// on the benchmark meshes, 1 % (hexahedra) to 5 % (tetrahedra) faster than 256
+constexpr int kGatherThreads = 128;
 
 template <bool TI>
 static int launch_fused_interior(salvus_problem *p, const HexInteriorUpdate &iu) {
@@ -890,7 +951,7 @@ static int step_fused_hex_interior(salvus_problem *p, bool store_a) {
     iu.ap = store_a ? F<float>(p->d_ap) : nullptr;
     iu.dt = (float)p->dt;
     iu.nsrc_elem = p->n_src_uelem;
-    iu.src_elem = p->d_src_uelem.as<int64_t>();
+    iu.src_elem = p->src_uelem;
     if ((rc = m->ti ? launch_fused_interior<true>(p, iu) : launch_fused_interior<false>(p, iu)))
       return rc;
   }
@@ -900,11 +961,9 @@ static int step_fused_hex_interior(salvus_problem *p, bool store_a) {
     auto go = [&](auto nt) {
       constexpr int N = decltype(nt)::value;
       source_fused_hex_kernel<N><<<1, 256, 0, p->stream>>>(
-          (int)p->srcs.size(), m->P, p->d_src_elem.as<int64_t>(), p->d_src_par.as<double>(),
-          p->d_src_wts.as<double>(), p->d_step.as<int64_t>(), p->dt, F<float>(p->d_r),
-          p->n_src_uelem, p->d_src_uelem.as<int64_t>(), m->d_conn.as<int32_t>(),
-          m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v),
-          store_a ? F<float>(p->d_ap) : nullptr, (float)p->dt);
+          m->P, F<float>(p->d_r), p->n_src_uelem, p->src_uelem,
+          m->d_conn.as<int32_t>(), m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v),
+          store_a ? F<float>(p->d_ap) : nullptr, (float)p->dt, source_terms(p));
     };
     switch (m->order) {
       case 2: go(std::integral_constant<int, 2>{}); break;
@@ -922,7 +981,8 @@ static int step_fused_hex_interior(salvus_problem *p, bool store_a) {
     gather_list_kernel<float, 3, 0><<<blocks_for(m->n_gnodes, 256), 256, 0, p->stream>>>(
         m->n_gnodes, m->d_gnodes.as<int32_t>(), m->d_inc_off.as<int32_t>(),
         m->d_inc_idx.as<int32_t>(), F<float>(p->d_r), m->d_mi32.as<float>(), F<float>(p->d_u),
-        F<float>(p->d_v), store_a ? F<float>(p->d_ap) : nullptr, nullptr, (float)p->dt);
+        F<float>(p->d_v), store_a ? F<float>(p->d_ap) : nullptr, nullptr, (float)p->dt,
+        source_terms(p), p->d_step.as<int64_t>());
     g_launches++;
     if ((rc = check_launch("gather update (shared nodes)"))) return rc;
   }
@@ -947,17 +1007,13 @@ static int step_fused_t(salvus_problem *p, bool store_a) {
   if ((rc = join_receivers(p))) return rc;  // the previous step's receivers
   if ((rc = launch_dirichlet<real, C>(p))) return rc;
   if ((rc = launch_coupling<real>(p))) return rc;
-  if ((rc = launch_sources<real, C>(p))) return rc;
   {
     ProfScope ps(p, K_UPDATE);
-    // 128-thread CTAs: measured against 64 / 256 / 512 on the benchmark
-    // meshes, 1 % (hexahedra) to 5 % (tetrahedra) faster than 256
-    constexpr int kGatherThreads = 128;
     gather_kernel<real, C, 0><<<blocks_for(m->G, kGatherThreads), kGatherThreads, 0, p->stream>>>(
         m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<real>(p->d_r),
         inv_mass<real>(p), F<real>(p->d_u), F<real>(p->d_v),
         store_a || m->physics == SALVUS_COUPLED2D ? F<real>(p->d_ap) : nullptr, nullptr,
-        (real)p->dt);
+        (real)p->dt, source_terms(p), p->d_step.as<int64_t>());
     g_launches++;
     if ((rc = check_launch("gather update"))) return rc;
   }
@@ -996,8 +1052,8 @@ static void launch_qb(const salvus_problem *p, cudaStream_t st, bool fuse) {
     bi.mi = m->d_mi32.as<float>();
     bi.w = F<float>(p->d_v);
     bi.dt = (float)p->dt;
-    bi.shot_off = p->srcs.empty() ? nullptr : p->d_shot_off.as<int32_t>();
-    bi.src_elem = p->d_src_elem.as<int64_t>();
+    bi.shot_off = p->srcs.empty() ? nullptr : p->shot_off;
+    bi.src_elem = p->src_elem;
     quad_acoustic_batched_kernel<N, SC, EPC, true><<<grid, SC * EPC, 0, st>>>(
         m->E, p->shots_pad, m->d_rec32.as<float>(), F<float>(p->d_u), F<float>(p->d_r),
         dmatrix<float>(m->basis), bi);
@@ -1038,30 +1094,32 @@ static int batched_stiffness(const salvus_problem *p, int cfg, cudaStream_t st, 
 }
 
 template <int SC, int NPB, int NPT = 1>
-static void launch_bg(const salvus_problem *p, cudaStream_t st, bool fuse) {
+static void launch_bg(const salvus_problem *p, cudaStream_t st, bool fuse, int64_t *step) {
   const salvus_mesh *m = p->mesh;
   const int64_t n = fuse ? m->n_gnodes : m->G;
   dim3 grid((unsigned)((n + NPB * NPT - 1) / (NPB * NPT)), (unsigned)(p->shots_pad / SC));
   batched_gather_update_kernel<SC, NPB, NPT><<<grid, SC * NPB, 0, st>>>(
       n, p->shots_pad, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(),
       F<float>(p->d_r), m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v), (float)p->dt,
-      fuse ? m->d_gnodes.as<int32_t>() : nullptr);
+      fuse ? m->d_gnodes.as<int32_t>() : nullptr, step);
 }
 
-static int batched_gather(const salvus_problem *p, int cfg, cudaStream_t st, bool fuse) {
+// step: the device step counter to advance (null: a timing run of the autotuner)
+static int batched_gather(const salvus_problem *p, int cfg, cudaStream_t st, bool fuse,
+                          int64_t *step) {
   switch (cfg) {
-    case 0: launch_bg<32, 4>(p, st, fuse); break;
-    case 1: launch_bg<32, 8>(p, st, fuse); break;
-    case 2: launch_bg<64, 2>(p, st, fuse); break;
-    case 3: launch_bg<64, 4>(p, st, fuse); break;
-    case 4: launch_bg<128, 1>(p, st, fuse); break;
-    case 5: launch_bg<128, 2>(p, st, fuse); break;
-    case 6: launch_bg<256, 1>(p, st, fuse); break;
-    case 7: launch_bg<32, 4, 2>(p, st, fuse); break;
-    case 8: launch_bg<64, 2, 2>(p, st, fuse); break;
-    case 9: launch_bg<128, 1, 2>(p, st, fuse); break;
-    case 10: launch_bg<128, 1, 4>(p, st, fuse); break;
-    case 11: launch_bg<256, 1, 2>(p, st, fuse); break;
+    case 0: launch_bg<32, 4>(p, st, fuse, step); break;
+    case 1: launch_bg<32, 8>(p, st, fuse, step); break;
+    case 2: launch_bg<64, 2>(p, st, fuse, step); break;
+    case 3: launch_bg<64, 4>(p, st, fuse, step); break;
+    case 4: launch_bg<128, 1>(p, st, fuse, step); break;
+    case 5: launch_bg<128, 2>(p, st, fuse, step); break;
+    case 6: launch_bg<256, 1>(p, st, fuse, step); break;
+    case 7: launch_bg<32, 4, 2>(p, st, fuse, step); break;
+    case 8: launch_bg<64, 2, 2>(p, st, fuse, step); break;
+    case 9: launch_bg<128, 1, 2>(p, st, fuse, step); break;
+    case 10: launch_bg<128, 1, 4>(p, st, fuse, step); break;
+    case 11: launch_bg<256, 1, 2>(p, st, fuse, step); break;
     default: return fail(SALVUS_E_INVALID, "bad gather config %d", cfg);
   }
   g_launches++;
@@ -1141,7 +1199,7 @@ static int autotune(salvus_problem *p) {
     int cg = -1;
     for (int c = 0; c < kNumGatherCfg && rc == SALVUS_OK; ++c) {
       if (p->shots_pad % kGatherCfg[c].sc) continue;
-      float t = time_it([&] { return batched_gather(p, c, p->stream, fuse); });
+      float t = time_it([&] { return batched_gather(p, c, p->stream, fuse, nullptr); });
       if (t < bg) { bg = t; cg = c; }
     }
     std::swap(p->d_u.ptr, su.ptr);
@@ -1173,8 +1231,8 @@ static int step_batched(salvus_problem *p) {
     // fused step: the source elements' interior nodes are finished here
     const bool fuse = batch_fusion(p) && m->order >= 2;
     batched_source_kernel<<<(total + threads - 1) / threads, threads, 0, p->stream>>>(
-        p->shots_pad, m->P, p->d_shot_off.as<int32_t>(), p->d_src_elem.as<int64_t>(),
-        p->d_src_par.as<double>(), p->d_src_wts.as<double>(), p->d_step.as<int64_t>(), p->dt,
+        p->shots_pad, m->P, p->shot_off, p->src_elem,
+        p->src_par, p->src_wts, p->d_step.as<int64_t>(), p->dt,
         F<float>(p->d_r), fuse ? m->n : 0, m->d_conn.as<int32_t>(), m->d_mi32.as<float>(),
         F<float>(p->d_u), F<float>(p->d_v), (float)p->dt);
     g_launches++;
@@ -1182,7 +1240,8 @@ static int step_batched(salvus_problem *p) {
   }
   {
     ProfScope ps(p, K_UPDATE);
-    if ((rc = batched_gather(p, p->tune_gather, p->stream, batch_fusion(p)))) return rc;
+    if ((rc = batched_gather(p, p->tune_gather, p->stream, batch_fusion(p),
+                             p->d_step.as<int64_t>()))) return rc;
   }
   ProfScope ps(p, K_REC);
   if (!p->recs.empty()) {
@@ -1193,8 +1252,6 @@ static int step_batched(salvus_problem *p) {
         p->d_seis.as<double>(), p->seis_cap, p->d_step.as<int64_t>());
     g_launches++;
   }
-  advance_step_kernel<<<1, 1, 0, p->stream>>>(p->d_step.as<int64_t>());
-  g_launches++;
   return check_launch("batched receivers");
 }
 
@@ -1238,11 +1295,10 @@ static int assemble_t(salvus_problem *p) {
   }
   if ((rc = launch_dirichlet<real, C>(p))) return rc;
   if ((rc = launch_coupling<real>(p))) return rc;
-  if ((rc = launch_sources<real, C>(p))) return rc;
   ProfScope ps(p, K_GATHER);
   gather_kernel<real, C, 1><<<blocks_for(m->G, 256), 256, 0, p->stream>>>(
       m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<real>(p->d_r), nullptr,
-      nullptr, nullptr, nullptr, F<real>(p->d_a), (real)0);
+      nullptr, nullptr, nullptr, F<real>(p->d_a), (real)0, source_terms(p));
   g_launches++;
   return check_launch("gather");
 }
@@ -1264,7 +1320,8 @@ static int newmark_t(salvus_problem *p) {
     ProfScope ps(p, K_NEWMARK);
     const int64_t N = p->mesh->G * C;
     newmark_kernel<real><<<blocks_for(N, 256), 256, 0, p->stream>>>(
-        N, F<real>(p->d_a), F<real>(p->d_u), F<real>(p->d_v), F<real>(p->d_ap), (real)p->dt);
+        N, F<real>(p->d_a), F<real>(p->d_u), F<real>(p->d_v), F<real>(p->d_ap), (real)p->dt,
+        p->d_step.as<int64_t>());
     g_launches++;
     if ((rc = check_launch("newmark"))) return rc;
   }
@@ -1361,17 +1418,18 @@ static int launch_finite_check(salvus_problem *p) {
 }
 
 // Hexahedron autotuner (FP32 elastic meshes of parallelepipeds, one shot):
-// times the plain step (stiffness, node gather/update) and, where the fused
-// interior form is admissible, that form, each with CTAs of 128 / (N+1)^2
-// elements and with twice as many, on zeroed scratch copies of u and w, and
-// keeps the fastest.  All of them give bitwise the same wavefield
-// (the same arithmetic per element and per node, in the same order), so the
-// choice changes only the time.  Results are cached per (order, elements,
-// nodes, anisotropy, admissible forms, device) for the process; the CTA
-// width belongs to the mesh, the form to the problem.
-// SALVUS_HEX_CONFIG="form,wide" fixes both; SALVUS_HEX_STEP still forces
-// the form.  Without room for the scratch fields the defaults (plain, 128 /
-// (N+1)^2) are kept.
+// times the plain step (stiffness, node gather/update) with CTAs of 128 /
+// (N+1)^2 elements and with twice as many, on zeroed scratch copies of u and
+// w, and keeps the faster.  Both give bitwise the same wavefield (the same
+// arithmetic per element and per node, in the same order), so the choice
+// changes only the time.  Results are cached per (order, elements, nodes,
+// anisotropy, device) for the process; the CTA width belongs to the mesh.
+// The fused interior form is not among the candidates: it lost on every mesh
+// measured (per step, plain against fused: 64^3 order 4 0.73 / 0.84 ms, 16^3
+// order 4 15.1 / 19.4 us, 18^3 order 5 anisotropic 35.6 / 52.1 us) and its
+// source launch and receivers stay on the critical path.
+// SALVUS_HEX_CONFIG="form,wide" fixes form and width; SALVUS_HEX_STEP forces
+// the form.  Without room for the scratch fields the default width is kept.
 static int tune_hex(salvus_problem *p) {
   if (p->hex_form >= 0) return SALVUS_OK;
   salvus_mesh *m = p->mesh;
@@ -1380,14 +1438,14 @@ static int tune_hex(salvus_problem *p) {
     p->hex_form = 0;
     return SALVUS_OK;
   }
-  const bool fusable = hex_fusion_admissible(p) && m->order >= 2 && m->order <= 6;
   struct Key {
     int order;
     int64_t E, G;
-    bool ti, fusable;
+    bool ti;
     int dev;
   };
   if (const char *env = std::getenv("SALVUS_HEX_CONFIG")) {
+    const bool fusable = hex_fusion_admissible(p) && m->order >= 2 && m->order <= 6;
     int a = -1, b = -1;
     if (std::sscanf(env, "%d,%d", &a, &b) == 2 && (a == 0 || (a == 1 && fusable)) &&
         (b == 0 || b == 1)) {
@@ -1398,14 +1456,14 @@ static int tune_hex(salvus_problem *p) {
   }
   // problems are prepared on several threads (the job server)
   static std::mutex cache_mu;
-  static std::vector<std::pair<Key, std::pair<int, int>>> cache;
+  static std::vector<std::pair<Key, int>> cache;
   {
     std::lock_guard<std::mutex> lk(cache_mu);
     for (auto &c : cache)
       if (c.first.order == m->order && c.first.E == m->E && c.first.G == m->G &&
-          c.first.ti == m->ti && c.first.fusable == fusable && c.first.dev == m->device) {
-        p->hex_form = c.second.first;
-        m->hex_wide = c.second.second;
+          c.first.ti == m->ti && c.first.dev == m->device) {
+        p->hex_form = 0;
+        m->hex_wide = c.second;
         return SALVUS_OK;
       }
   }
@@ -1420,70 +1478,49 @@ static int tune_hex(salvus_problem *p) {
   }
   SALVUS_CUDA(cudaMemsetAsync(su.ptr, 0, nf, p->stream));
   SALVUS_CUDA(cudaMemsetAsync(sv.ptr, 0, nf, p->stream));
-  std::swap(p->d_u.ptr, su.ptr);
-  std::swap(p->d_v.ptr, sv.ptr);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   int rc = SALVUS_OK;
-  // one step of either form without sources and receivers (the same in both)
-  auto sequence = [&](int form) -> int {
+  // one step without sources and receivers (the same for both widths)
+  auto sequence = [&]() -> int {
     int r;
-    if (form == 0) {
-      if ((r = launch_stiffness<float>(m, records<float>(p), F<float>(p->d_u), F<float>(p->d_r),
-                                       p->stream, p->d_err.as<int>(), p->wait_limit, 0)))
-        return r;
-      gather_kernel<float, 3, 0><<<blocks_for(m->G, 256), 256, 0, p->stream>>>(
-          m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<float>(p->d_r),
-          m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v), nullptr, nullptr, (float)p->dt);
-    } else {
-      HexInteriorUpdate iu{};
-      iu.mi = m->d_mi32.as<float>();
-      iu.w = F<float>(p->d_v);
-      iu.dt = (float)p->dt;
-      if ((r = m->ti ? launch_fused_interior<true>(p, iu) : launch_fused_interior<false>(p, iu)))
-        return r;
-      gather_list_kernel<float, 3, 0><<<blocks_for(m->n_gnodes, 256), 256, 0, p->stream>>>(
-          m->n_gnodes, m->d_gnodes.as<int32_t>(), m->d_inc_off.as<int32_t>(),
-          m->d_inc_idx.as<int32_t>(), F<float>(p->d_r), m->d_mi32.as<float>(), F<float>(p->d_u),
-          F<float>(p->d_v), nullptr, nullptr, (float)p->dt);
-    }
+    if ((r = launch_stiffness<float>(m, records<float>(p), su.as<float>(), F<float>(p->d_r),
+                                     p->stream, p->d_err.as<int>(), p->wait_limit, 0)))
+      return r;
+    gather_kernel<float, 3, 0><<<blocks_for(m->G, kGatherThreads), kGatherThreads, 0, p->stream>>>(
+        m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<float>(p->d_r),
+        m->d_mi32.as<float>(), su.as<float>(), sv.as<float>(), nullptr, nullptr, (float)p->dt);
     g_launches++;
     return check_launch("hexahedron autotuner");
   };
   float best = 1e30f;
-  int bf = 0, bw = 0;
+  int bw = 0;
   for (int w = 0; w < 2 && rc == SALVUS_OK; ++w) {
     m->hex_wide = w;
-    for (int f = 0; f < (fusable ? 2 : 1) && rc == SALVUS_OK; ++f) {
-      if ((rc = sequence(f))) break;  // first launch (attributes, caches)
-      float t = 1e30f;
-      for (int rep = 0; rep < 3 && rc == SALVUS_OK; ++rep) {
-        cudaEventRecord(e0, p->stream);
-        for (int k = 0; k < 4 && rc == SALVUS_OK; ++k) rc = sequence(f);
-        cudaEventRecord(e1, p->stream);
-        cudaEventSynchronize(e1);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
-        t = std::min(t, ms);
-      }
-      if (rc == SALVUS_OK && t < best) {
-        best = t;
-        bf = f;
-        bw = w;
-      }
+    if ((rc = sequence())) break;  // first launch (attributes, caches)
+    float t = 1e30f;
+    for (int rep = 0; rep < 3 && rc == SALVUS_OK; ++rep) {
+      cudaEventRecord(e0, p->stream);
+      for (int k = 0; k < 4 && rc == SALVUS_OK; ++k) rc = sequence();
+      cudaEventRecord(e1, p->stream);
+      cudaEventSynchronize(e1);
+      float ms = 0;
+      cudaEventElapsedTime(&ms, e0, e1);
+      t = std::min(t, ms);
+    }
+    if (rc == SALVUS_OK && t < best) {
+      best = t;
+      bw = w;
     }
   }
   cudaStreamSynchronize(p->stream);
-  std::swap(p->d_u.ptr, su.ptr);
-  std::swap(p->d_v.ptr, sv.ptr);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   m->hex_wide = bw;
   if (rc) return rc;
-  p->hex_form = bf;
   std::lock_guard<std::mutex> lk(cache_mu);
-  cache.push_back({{m->order, m->E, m->G, m->ti, fusable, m->device}, {bf, bw}});
+  cache.push_back({{m->order, m->E, m->G, m->ti, m->device}, bw});
   return SALVUS_OK;
 }
 
@@ -1624,9 +1661,9 @@ static int group_fill(salvus_group *g) {
     s.step = p->d_step.as<int64_t>();
     s.nsrc = (int)p->srcs.size();
     s.nrec = (int)p->recs.size();
-    s.src_elem = p->d_src_elem.as<int64_t>();
-    s.src_par = p->d_src_par.as<double>();
-    s.src_wts = p->d_src_wts.as<double>();
+    s.src_par = p->src_par;
+    s.src = source_terms(p);
+    s.stf = p->stf;
     s.rec_elem = p->d_rec_elem.as<int64_t>();
     s.rec_l = p->d_rec_l.as<double>();
     s.seis = p->d_seis.as<double>();
@@ -1636,7 +1673,7 @@ static int group_fill(salvus_group *g) {
     s.b_rec = br;
     bs += group_stiff_blocks(m);
     bg += (m->G + 255) / 256;
-    br += s.nrec;
+    br += s.nrec + (s.nsrc > 0 ? 1 : 0);
   }
   g->n_stiff = bs;
   g->n_gather = bg;
@@ -1651,7 +1688,8 @@ static int group_fill(salvus_group *g) {
       const salvus_mesh *mk = g->members[k]->mesh;
       std::fill(o + sk.b_stiff, o + sk.b_stiff + group_stiff_blocks(mk), (int32_t)k);
       std::fill(o + bs + sk.b_gather, o + bs + sk.b_gather + (mk->G + 255) / 256, (int32_t)k);
-      std::fill(o + bs + bg + sk.b_rec, o + bs + bg + sk.b_rec + sk.nrec, (int32_t)k);
+      std::fill(o + bs + bg + sk.b_rec, o + bs + bg + sk.b_rec + sk.nrec + (sk.nsrc > 0 ? 1 : 0),
+                (int32_t)k);
     }
   }
   if ((rc = group_upload(g->d_owner, g->owner.data(), sizeof(int32_t) * g->owner.size(), g->stream)))
@@ -1850,23 +1888,19 @@ static int group_partitioned(salvus_group *g, bool launch, bool store_a) {
 static int group_step(salvus_group *g, bool store_a) {
   if (g->partitioned) return group_partitioned(g, true, store_a);
   if (!g->stages) return group_persistent(g, store_a);
-  const int J = (int)g->members.size();
   const int P = g->m0->P;
   const GroupSlot *slots = g->d_slots.as<GroupSlot>();
   int rc;
   const int32_t *own = g->d_owner.as<int32_t>();
   if ((rc = group_stiffness(g->m0, slots, own, g->n_stiff, g->stream))) return rc;
-  if (g->c == 1) group_source<1><<<J, 256, 0, g->stream>>>(slots, P);
-  else group_source<3><<<J, 256, 0, g->stream>>>(slots, P);
   if (g->c == 1) group_gather_update<1><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff, store_a);
   else group_gather_update<3><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff, store_a);
   if (g->n_rec > 0) {
     const int32_t *own_rec = own + g->n_stiff + g->n_gather;
-    if (g->c == 1) group_receivers<1><<<(unsigned)g->n_rec, kRecThreads, 0, g->stream>>>(slots, own_rec, P);
-    else group_receivers<3><<<(unsigned)g->n_rec, kRecThreads, 0, g->stream>>>(slots, own_rec, P);
+    if (g->c == 1) group_step_tail<1><<<(unsigned)g->n_rec, kRecThreads, 0, g->stream>>>(slots, own_rec, P);
+    else group_step_tail<3><<<(unsigned)g->n_rec, kRecThreads, 0, g->stream>>>(slots, own_rec, P);
   }
-  group_advance<<<1, 256, 0, g->stream>>>(slots, J);
-  g_launches += g->n_rec > 0 ? 4 : 3;
+  g_launches += g->n_rec > 0 ? 2 : 1;
   return check_launch("group step");
 }
 
@@ -2235,6 +2269,7 @@ int salvus_problem_set_dt(salvus_problem *p, double dt) {
     drop_graph(p);
     SALVUS_CUDA(cudaSetDevice(p->mesh->device));
     if (int rc = velocity_form(p, false)) return rc;  // w belongs to the old step
+    p->stf_ready = false;
   }
   p->dt = dt;
   p->dt_set = true;
@@ -2607,6 +2642,7 @@ int salvus_assemble(salvus_problem *p) {
   if (rc) return rc;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
   if ((rc = velocity_form(p, true))) return rc;  // the coupling terms read v through w
+  if ((rc = sources_ready(p))) return rc;
   return by_components(p->c, [&](auto cc) {
     constexpr int C = decltype(cc)::value;
     return p->prec == SALVUS_FP32 ? assemble_t<float, C>(p) : assemble_t<double, C>(p);
@@ -2645,7 +2681,7 @@ int salvus_step(salvus_problem *p) {
   int rc = ready(p);
   if (rc) return rc;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
-  if ((rc = velocity_form(p, true))) return rc;
+  if ((rc = velocity_form(p, true)) || (rc = sources_ready(p))) return rc;
   rc = step_fused(p, true);
   if (rc == SALVUS_OK) p->step++;
   if (rc == SALVUS_OK && p->step % kFiniteEvery == 0) rc = launch_finite_check(p);
@@ -2755,7 +2791,7 @@ int salvus_run(salvus_problem *p, int64_t n_steps, int32_t mode) {
     return fail(SALVUS_E_INVALID, "unknown run mode %d", mode);
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
   if ((rc = rec_stream_ready(p))) return rc;
-  if (n_steps > 0 && (rc = velocity_form(p, true))) return rc;
+  if (n_steps > 0 && ((rc = velocity_form(p, true)) || (rc = sources_ready(p)))) return rc;
   return run_steps(p, n_steps, mode);
 }
 
@@ -3032,8 +3068,11 @@ int salvus_group_run(salvus_group *g, int64_t n_steps) {
   if (!g) return fail(SALVUS_E_INVALID, "null group");
   if (n_steps < 0) return fail(SALVUS_E_INVALID, "negative step count");
   SALVUS_CUDA(cudaSetDevice(g->m0->device));
-  for (auto *p : g->members)
-    if (int rc = velocity_form(p, true)) return rc;
+  for (auto *p : g->members) {
+    int rc = ready(p);
+    if (rc || (rc = velocity_form(p, true)) || (rc = sources_ready(p))) return rc;
+    if (!g->stages && n_steps > 0) p->stf_ready = false;  // these forms have no tail
+  }
   // order the group after every member's pending work
   for (size_t k = 0; k < g->members.size(); ++k) {
     SALVUS_CUDA(cudaEventRecord(g->member_ev[k], g->members[k]->stream));
@@ -3064,7 +3103,7 @@ int salvus_group_run(salvus_group *g, int64_t n_steps) {
   int64_t done = 0;
   while (g->graph && n_steps - done >= g->graph_steps) {
     SALVUS_CUDA(cudaGraphLaunch(g->graph, g->stream));
-    g_launches += (int64_t)g->graph_steps * (g->stages ? (g->n_rec > 0 ? 5 : 4) : 1);
+    g_launches += (int64_t)g->graph_steps * (g->stages ? (g->n_rec > 0 ? 3 : 2) : 1);
     done += g->graph_steps;
   }
   for (; done < n_steps; ++done)

@@ -189,9 +189,20 @@ struct salvus_problem {
     std::vector<double> wts;  // [P][c]
   };
   std::vector<Src> srcs;
-  salvus::DeviceBuffer d_src_elem, d_src_par, d_src_wts;
-  salvus::DeviceBuffer d_src_uelem;  // distinct source elements (fused hexahedron step)
+  // everything the kernels read of the sources, in one allocation (d_src):
+  // per source its element, [f0, t0, amplitude] and weights; batched: the
+  // shots' offsets; the distinct source elements (fused hexahedron step);
+  // SourceTerms (kernels_step.cuh): the node tiles, their entries and the
+  // source-time functions of the coming step (stf_ready: stf holds them for
+  // the step that the device counter stands at)
+  salvus::DeviceBuffer d_src;
+  const int64_t *src_elem = nullptr, *src_uelem = nullptr;
+  const double *src_par = nullptr, *src_wts = nullptr;
+  const int32_t *shot_off = nullptr, *src_tile = nullptr;
+  const int4 *src_node = nullptr;
+  double *stf = nullptr;
   int n_src_uelem = 0;
+  bool stf_ready = false;
   bool src_dirty = true;
   // receivers
   struct Rec {
@@ -207,7 +218,6 @@ struct salvus_problem {
   // shot batching (shots > 1): fields are [G][c][S_pad]; d_v holds the
   // half-step velocity w = v + dt/2 a_; sources grouped by shot
   int shots_pad = 1;
-  salvus::DeviceBuffer d_shot_off;
   int tune_stiff = -1, tune_gather = -1;  // autotuner choices (indices)
   int hex_form = -1;  // hexahedron step form: 0 plain, 1 fused interior update (-1 untuned)
   // graphs

@@ -182,7 +182,8 @@ batched_gather_update_kernel(int64_t G, int S, const int32_t *__restrict__ off,
                              const int32_t *__restrict__ idx, const float *__restrict__ r,
                              const float *__restrict__ mi, float *__restrict__ u,
                              float *__restrict__ w, float dt,
-                             const int32_t *__restrict__ nodes = nullptr) {
+                             const int32_t *__restrict__ nodes, int64_t *__restrict__ step) {
+  if (step && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *step += 1;
   const int ny = threadIdx.x / SC, lane = threadIdx.x - ny * SC;
   const int64_t g0 = ((int64_t)blockIdx.x * NPB + ny) * NPT;
   const int s = blockIdx.y * SC + lane;
@@ -238,7 +239,8 @@ batched_gather_update_kernel(int64_t G, int S, const int32_t *__restrict__ off,
 }
 
 // Receivers of every shot: block = receiver, thread = shot; FP64 Kahan over
-// the element points.  seis[(s * R + rec) * cap + step % cap].
+// the element points.  seis[(s * R + rec) * cap + n % cap] after step n, the
+// one just completed (*step - 1).
 __global__ void batched_receiver_kernel(int S, int R, int P, const int64_t *__restrict__ elem,
                                         const double *__restrict__ lw,
                                         const int32_t *__restrict__ conn,
@@ -246,7 +248,7 @@ __global__ void batched_receiver_kernel(int S, int R, int P, const int64_t *__re
                                         int64_t cap, const int64_t *__restrict__ step) {
   const int rc = blockIdx.x;
   const int64_t e = elem[rc];
-  const int64_t slot = *step % cap;
+  const int64_t slot = (*step - 1) % cap;
   for (int s = threadIdx.x; s < S; s += blockDim.x) {
     double acc = 0.0, comp = 0.0;
     for (int p = 0; p < P; ++p) {

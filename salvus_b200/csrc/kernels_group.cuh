@@ -5,7 +5,8 @@
 // gets alone.
 //
 // Per step, per member, the single-problem order (abi.cu step_fused_t):
-// stiffness, source, gather/update, receivers, step-counter advance.
+// stiffness, gather/update with the sources, receivers (the single-launch
+// forms evaluate the source-time functions in an item of their own).
 //
 // group_persistent_step: ONE launch per step for the whole group.  Resident
 // CTAs take work items from a queue, all members' stiffness tiles first, then
@@ -37,8 +38,9 @@ struct GroupSlot {
   double dtd;
   int64_t *step;
   int nsrc, nrec;
-  const int64_t *src_elem;
-  const double *src_par, *src_wts;
+  const double *src_par;
+  SourceTerms src;
+  double *stf;
   const int64_t *rec_elem;
   const double *rec_l;
   double *seis;
@@ -81,32 +83,29 @@ group_hex_elastic_stiffness(const GroupSlot *__restrict__ slots,
   group_hex_body<N, EPB>(m, blockIdx.x - m.b_stiff, Dm);
 }
 
-// one CTA per member
-template <int C>
-__global__ void group_source(const GroupSlot *__restrict__ slots, int P) {
-  const GroupSlot &m = slots[blockIdx.x];
-  if (m.nsrc > 0) source_body<float, C>(m.nsrc, P, m.src_elem, m.src_par, m.src_wts, m.step, m.dtd, m.r);
-}
-
 template <int C>
 __global__ void group_gather_update(const GroupSlot *__restrict__ slots,
                                     const int32_t *__restrict__ owner, bool store_a) {
   const GroupSlot &m = slots[owner[blockIdx.x]];
   const int64_t g = (blockIdx.x - m.b_gather) * (int64_t)blockDim.x + threadIdx.x;
+  if (g == 0) *m.step += 1;
   gather_body<float, C, 0>(g, m.G, m.inc_off, m.inc_idx, m.r, m.mi, m.u, m.w,
-                           store_a ? m.ap : nullptr, nullptr, m.dt);
+                           store_a ? m.ap : nullptr, nullptr, m.dt, m.src);
 }
 
+// step_tail_kernel of all members: per member its receivers, then (members
+// with sources) one CTA for the source-time functions
 template <int C>
 __global__ void __launch_bounds__(kRecThreads)
-group_receivers(const GroupSlot *__restrict__ slots, const int32_t *__restrict__ owner, int P) {
+group_step_tail(const GroupSlot *__restrict__ slots, const int32_t *__restrict__ owner, int P) {
   const GroupSlot &m = slots[owner[blockIdx.x]];
-  receiver_body<float, C>((int)(blockIdx.x - m.b_rec), P, m.rec_elem, m.rec_l, m.conn, m.u, m.seis,
-                          m.cap, m.step);
-}
-
-__global__ void group_advance(const GroupSlot *__restrict__ slots, int J) {
-  for (int s = threadIdx.x; s < J; s += blockDim.x) *slots[s].step += 1;
+  const int b = (int)(blockIdx.x - m.b_rec);
+  const int64_t n = *m.step;
+  if (b < m.nrec) {
+    receiver_body<float, C>(b, P, m.rec_elem, m.rec_l, m.conn, m.u, m.seis, m.cap, n - 1);
+    return;
+  }
+  source_times(m.nsrc, m.src_par, n, m.dtd, m.stf);
 }
 
 // ---------------------------------------------------------------------------
@@ -196,15 +195,15 @@ group_persistent_step(const GroupSlot *__restrict__ slots, const GroupCounts *__
         }
         break;
       case GI_SRC:
-        if (m.nsrc > 0) source_body<float, C>(m.nsrc, P, m.src_elem, m.src_par, m.src_wts, m.step, m.dtd, m.r);
+        source_times(m.nsrc, m.src_par, *m.step, m.dtd, m.stf);
         break;
       case GI_GATHER:
         for (int b = w.first; b < w.first + w.count; ++b)
           gather_body<float, C, 0, true>((int64_t)b * blockDim.x + t, m.G, m.inc_off, m.inc_idx, m.r, m.mi,
-                                   m.u, m.w, store_a ? m.ap : nullptr, nullptr, m.dt);
+                                   m.u, m.w, store_a ? m.ap : nullptr, nullptr, m.dt, m.src);
         break;
       case GI_REC:
-        receiver_body<float, C, true>(w.first, P, m.rec_elem, m.rec_l, m.conn, m.u, m.seis, m.cap, m.step);
+        receiver_body<float, C, true>(w.first, P, m.rec_elem, m.rec_l, m.conn, m.u, m.seis, m.cap, *m.step);
         break;
       default:
         if (t == 0) *m.step += 1;
@@ -298,8 +297,7 @@ group_partitioned_step(const GroupSlot *__restrict__ slots, const GroupPart *__r
   bool ok = true;
   if (b == 0) {
     ok = member_wait(&gb->stiff_done, nb);
-    if (ok && m.nsrc > 0)
-      source_body<float, C>(m.nsrc, P, m.src_elem, m.src_par, m.src_wts, m.step, m.dtd, m.r);
+    if (ok) source_times(m.nsrc, m.src_par, *m.step, m.dtd, m.stf);
     __syncthreads();
     if (t == 0) {
       __threadfence();
@@ -311,13 +309,13 @@ group_partitioned_step(const GroupSlot *__restrict__ slots, const GroupPart *__r
   if (ok)
     for (int k = b; k < pt.n_gather; k += nb)
       gather_body<float, C, 0, true>((int64_t)k * 128 + t, m.G, m.inc_off, m.inc_idx, m.r, m.mi,
-                                     m.u, m.w, store_a ? m.ap : nullptr, nullptr, m.dt);
+                                     m.u, m.w, store_a ? m.ap : nullptr, nullptr, m.dt, m.src);
   arrive(&gb->gather_done);
   ok = ok && member_wait(&gb->gather_done, nb);
   // receivers
   if (ok)
     for (int k = b; k < m.nrec; k += nb)
-      receiver_body<float, C, true>(k, P, m.rec_elem, m.rec_l, m.conn, m.u, m.seis, m.cap, m.step);
+      receiver_body<float, C, true>(k, P, m.rec_elem, m.rec_l, m.conn, m.u, m.seis, m.cap, *m.step);
   arrive(&gb->rec_done);
   if (b == 0) {
     ok = ok && member_wait(&gb->rec_done, nb);

@@ -18,8 +18,8 @@
 // (newmark_point) -- and writes element-local residuals only for the points
 // on the element's faces, which the node gather then assembles over the
 // shared nodes alone.  In the few elements that hold a source the interior
-// residuals are written too; the source kernel adds the source terms in
-// attach order and then finishes those nodes (source_interior_body).  Every operation and its order is the one of the
+// residuals are written too; the source kernel adds the source terms and
+// finishes those nodes (source_fused_hex_kernel).  Every operation and its order is the one of the
 // unfused sequence (stiffness, sources, gather, update), so the two forms
 // give bitwise the same wavefield.  In the fused form u is written for
 // interior nodes during the launch, so u is read with coherent loads (the
@@ -37,7 +37,7 @@ namespace salvus {
 
 // Interior-node update of the fused step: Newmark state, inverse mass, and
 // the elements that hold a source (their interior nodes are finished by the
-// source kernel after the source terms are added: source_interior_body).
+// source kernel, which adds the source terms).
 struct HexInteriorUpdate {
   const float *mi;
   float *w, *ap;  // ap: null unless this step stores a_
@@ -225,36 +225,39 @@ __device__ __forceinline__ void elastic_hex_affine_body(
   }
 }
 
-// Source kernel of the fused step (one CTA): the source terms in attach
-// order into the element-local residual (source_body), then the interior
-// nodes of the distinct source elements -- which the fused stiffness kernel
-// left to it -- with the one-term assembly 0 + r, the inverse mass and the
-// Newmark update: the arithmetic of the node gather, so the result is the
-// unfused sequence's.
+// Source kernel of the fused step (one CTA): the interior nodes of the
+// source elements -- which the fused stiffness kernel left to it -- with the
+// one-term assembly 0 + r, the source terms (add_sources), the inverse mass
+// and the Newmark update: the arithmetic of the node gather, so the result is
+// the unfused sequence's.
 template <int N>
-__global__ void source_fused_hex_kernel(int nsrc, int P, const int64_t *__restrict__ elem,
-                                       const double *__restrict__ par,
-                                       const double *__restrict__ wts,
-                                       const int64_t *__restrict__ step, double dtd,
-                                       float *__restrict__ r, int nse,
+__global__ void source_fused_hex_kernel(int P, const float *__restrict__ r, int nse,
                                        const int64_t *__restrict__ src_elems,
                                        const int32_t *__restrict__ conn,
                                        const float *__restrict__ mi, float *__restrict__ u,
-                                       float *__restrict__ w, float *__restrict__ ap, float dt) {
-  source_body<float, 3>(nsrc, P, elem, par, wts, step, dtd, r);  // ends with __syncthreads
+                                       float *__restrict__ w, float *__restrict__ ap, float dt,
+                                       SourceTerms src) {
   constexpr int n = N + 1, m = N - 1, NI = m * m * m;
-  for (int t = threadIdx.x; t < nse * NI * 3; t += blockDim.x) {
-    const int se = t / (NI * 3), rem = t - se * NI * 3, q = rem / 3, c = rem - q * 3;
+  for (int t = threadIdx.x; t < nse * NI; t += blockDim.x) {
+    const int se = t / NI, q = t - se * NI;
     const int i = 1 + q % m, j = 1 + (q / m) % m, k = 1 + q / (m * m);
     const int64_t e = src_elems[se];
     const int pt = i + n * j + n * n * k;
-    const int64_t g = conn[e * P + pt], x = g * 3 + c;
-    float uo = u[x], wo = w[x];
-    const float an = mul_rn(add_rn(0.f, r[(e * P + pt) * 3 + c]), mi[g]);
-    newmark_point<float>(an, wo, uo, dt);
-    u[x] = uo;
-    w[x] = wo;
-    if (ap) ap[x] = an;
+    const int32_t g = conn[e * P + pt];
+    float acc[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) acc[c] = add_rn(0.f, r[(e * P + pt) * 3 + c]);
+    add_sources<float, 3, false>(src.node[src.tile[g / kSrcTile] + g % kSrcTile], src, acc);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int64_t x = (int64_t)g * 3 + c;
+      float uo = u[x], wo = w[x];
+      const float an = mul_rn(acc[c], mi[g]);
+      newmark_point<float>(an, wo, uo, dt);
+      u[x] = uo;
+      w[x] = wo;
+      if (ap) ap[x] = an;
+    }
   }
 }
 

@@ -67,6 +67,47 @@ __global__ void velocity_kernel(int64_t N, const real *__restrict__ w, const rea
   if (i < N) out[i] = (double)half_step_velocity<real>(w[i], ap[i], hdt);
 }
 
+// Source terms of a single-shot problem: added by the node gather to a
+// node's assembled residual (Problem.cpp:188-200: a = f - K u).  A kernel of
+// its own between the stiffness and the gather is a few threads' work at the
+// price of a launch and of its latency on the critical path: about 2 of the
+// 7.5 us that a step of a 40 x 40 order-4 quadrilateral mesh took (B200).
+// The gather finds the few nodes concerned through a table by tile of
+// kSrcTile nodes: tile[b] is -1, or where the tile's kSrcTile entries begin
+// in `node`: {x, y, z, w} = weights of source y at this node (index into
+// wts / C), first source y, z sources (0: none; an element's sources are
+// adjacent, in attach order, their weights P apart), w: the node's entry for
+// another source element or -1.  Two loads lead to the weights, as two lead
+// to the residual, and the sum needs no residual slot: adding the terms to
+// the incident residual of their element instead kept all eight points'
+// indices and residuals live (48 -> 72 registers for 3 components).
+// stf holds the source-time functions of the coming step, which the receiver
+// launch of the step before evaluates (step_tail_kernel).
+constexpr int kSrcTile = 128;
+struct SourceTerms {
+  const int32_t *tile = nullptr;  // null: no sources
+  const int4 *node;
+  const double *wts;  // [source][P][C]
+  const double *stf;  // [source]
+  int P;
+};
+
+// kInKernel: stf was written earlier in the same launch (coherent loads).
+template <typename real, int C, bool kInKernel>
+__device__ __forceinline__ void add_sources(int4 at, const SourceTerms &src, real (&acc)[C]) {
+  for (;;) {
+    for (int32_t s = 0; s < at.z; ++s) {
+      const double *sp = src.stf + at.y + s;
+      const double stf = kInKernel ? __ldca(sp) : *sp;
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        acc[c] = add_rn(acc[c], (real)__dmul_rn(src.wts[(at.x + (int64_t)s * src.P) * C + c], stf));
+    }
+    if (at.w < 0) return;
+    at = src.node[at.w];
+  }
+}
+
 // mode 0: fused  a = mi * sum(r); Newmark update of (u, w); a_ = a is stored
 //         when ap is not null (the last step of a run: later steps never read
 //         it, only callers do)
@@ -79,7 +120,8 @@ __device__ __forceinline__ void gather_body(int64_t g, int64_t G, const int32_t 
                                             const real *__restrict__ r,
                                             const real *__restrict__ mi, real *__restrict__ u,
                                             real *__restrict__ w, real *__restrict__ ap,
-                                            real *__restrict__ a, real dt) {
+                                            real *__restrict__ a, real dt,
+                                            const SourceTerms &src = SourceTerms()) {
   if (g >= G) return;
   // Newmark operands first: they do not depend on the gather, so their loads
   // overlap the dependent index -> residual chain below.
@@ -96,6 +138,7 @@ __device__ __forceinline__ void gather_body(int64_t g, int64_t G, const int32_t 
 #pragma unroll
   for (int c = 0; c < C; ++c) acc[c] = 0;
   const int32_t q0 = off[g], q1 = off[g + 1];
+  const int32_t src_at = src.tile ? src.tile[g / kSrcTile] : -1;
   const int cnt = q1 - q0;
   constexpr int kFast = 8;  // hexahedral / quadrilateral valence bound
   if (cnt <= kFast) {
@@ -143,6 +186,8 @@ __device__ __forceinline__ void gather_body(int64_t g, int64_t G, const int32_t 
         }
     }
   }
+  if (src_at >= 0)
+    add_sources<real, C, kInKernelR>(src.node[src_at + g % kSrcTile], src, acc);
   if constexpr (MODE == 1) {
 #pragma unroll
     for (int c = 0; c < C; ++c) a[g * C + c] = acc[c];
@@ -164,9 +209,12 @@ __global__ void gather_kernel(int64_t G, const int32_t *__restrict__ off,
                               const int32_t *__restrict__ idx, const real *__restrict__ r,
                               const real *__restrict__ mi, real *__restrict__ u,
                               real *__restrict__ w, real *__restrict__ ap, real *__restrict__ a,
-                              real dt) {
+                              real dt, SourceTerms src = SourceTerms(),
+                              int64_t *__restrict__ step = nullptr) {
+  // step counter (steps completed): nothing else of the launch reads it
+  if (step && blockIdx.x == 0 && threadIdx.x == 0) *step += 1;
   gather_body<real, C, MODE>((int64_t)blockIdx.x * blockDim.x + threadIdx.x, G, off, idx, r, mi, u,
-                             w, ap, a, dt);
+                             w, ap, a, dt, src);
 }
 
 // The gather / update over a list of nodes (the shared nodes of a fused
@@ -177,10 +225,13 @@ __global__ void gather_list_kernel(int64_t n, const int32_t *__restrict__ nodes,
                                    const int32_t *__restrict__ idx, const real *__restrict__ r,
                                    const real *__restrict__ mi, real *__restrict__ u,
                                    real *__restrict__ w, real *__restrict__ ap,
-                                   real *__restrict__ a, real dt) {
+                                   real *__restrict__ a, real dt,
+                                   SourceTerms src = SourceTerms(),
+                                   int64_t *__restrict__ step = nullptr) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (step && t == 0) *step += 1;
   if (t >= n) return;
-  gather_body<real, C, MODE>(nodes[t], INT64_MAX, off, idx, r, mi, u, w, ap, a, dt);
+  gather_body<real, C, MODE>(nodes[t], INT64_MAX, off, idx, r, mi, u, w, ap, a, dt, src);
 }
 
 // Blow-up detection: any NaN / Inf among n values sets the problem's device
@@ -244,8 +295,10 @@ __global__ void inverse_mass_kernel(int64_t G, const real *__restrict__ mi, real
 
 template <typename real>
 __global__ void newmark_kernel(int64_t N, const real *__restrict__ a, real *__restrict__ u,
-                               real *__restrict__ w, real *__restrict__ ap, real dt) {
+                               real *__restrict__ w, real *__restrict__ ap, real dt,
+                               int64_t *__restrict__ step) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *step += 1;
   if (i >= N) return;
   const real an = a[i];
   real wv = w[i], uv = u[i];
@@ -261,35 +314,19 @@ __device__ __forceinline__ double ricker_dev(double t, double f0, double t0, dou
   return amp * ((1 - 2 * factor) * exp(-1 * factor));
 }
 
-// Sources in attach order, one CTA; adds w_{p,c} * stf(t_n) into the
-// element-local residual of the source element.  src_par = [f0, t0, amp].
-template <typename real, int C>
-__device__ __forceinline__ void source_body(int nsrc, int P, const int64_t *__restrict__ elem,
-                                            const double *__restrict__ par,
-                                            const double *__restrict__ wts,
-                                            const int64_t *__restrict__ step, double dt,
-                                            real *__restrict__ r) {
-  const double t = (double)(*step) * dt;
-  for (int s = 0; s < nsrc; ++s) {
-    const double stf = ricker_dev(t, par[3 * s], par[3 * s + 1], par[3 * s + 2]);
-    const int64_t base = elem[s] * P * C;
-    for (int q = threadIdx.x; q < P * C; q += blockDim.x)
-      r[base + q] += (real)(wts[(int64_t)s * P * C + q] * stf);
-    __syncthreads();
-  }
-}
-
-template <typename real, int C>
-__global__ void source_kernel(int nsrc, int P, const int64_t *__restrict__ elem,
-                              const double *__restrict__ par, const double *__restrict__ wts,
-                              const int64_t *__restrict__ step, double dt, real *__restrict__ r) {
-  source_body<real, C>(nsrc, P, elem, par, wts, step, dt, r);
+// Source-time functions of step n into stf, by the threads of one CTA.
+// par = [f0, t0, amplitude] of each source.
+__device__ __forceinline__ void source_times(int nsrc, const double *__restrict__ par, int64_t n,
+                                             double dt, double *__restrict__ stf) {
+  for (int s = threadIdx.x; s < nsrc; s += blockDim.x)
+    stf[s] = ricker_dev((double)n * dt, par[3 * s], par[3 * s + 1], par[3 * s + 2]);
 }
 
 // Receivers: one CTA per receiver, one thread per element point (strided);
 // each thread keeps a Kahan-compensated FP64 partial per component, then a
-// fixed-order tree combines the partials (deterministic).
-// seis[(rec*C + c)*cap + step % cap] = sum_p l_p u_p.
+// fixed-order tree combines the partials (deterministic): across each warp
+// by shuffles, then the warps' sums in order.
+// seis[(rec*C + c)*cap + n % cap] = sum_p l_p u_p after step n.
 // kInKernelU: u was written earlier in the same launch (fused group steps),
 // so it is read with a coherent load (ld.global.ca, ordered by the waits'
 // fences), never through the non-coherent read-only path (ld.global.nc),
@@ -300,17 +337,15 @@ __device__ __forceinline__ void receiver_body(int rc, int P, const int64_t *__re
                                               const double *__restrict__ lw,
                                               const int32_t *__restrict__ conn,
                                               const real *__restrict__ u,
-                                              double *__restrict__ seis, int64_t cap,
-                                              const int64_t *__restrict__ step) {
-  __shared__ double part[C][kRecThreads];
-  // CTAs wider than kRecThreads (grouped persistent steps) keep their extra
-  // threads idle here but in every barrier
+                                              double *__restrict__ seis, int64_t cap, int64_t n) {
+  constexpr int kWarps = kRecThreads / 32;
+  __shared__ double part[C][kWarps];
   const int t = threadIdx.x;
-  const int64_t e = elem[rc];
+  const int64_t e = elem[rc], col = t < C ? n % cap : 0;
   double s[C], comp[C];
 #pragma unroll
   for (int c = 0; c < C; ++c) s[c] = comp[c] = 0.0;
-  for (int p = t; p < P && t < kRecThreads; p += kRecThreads) {
+  for (int p = t; p < P; p += kRecThreads) {
     const double l = lw[(int64_t)rc * P + p];
     const int64_t node = conn[e * P + p];
 #pragma unroll
@@ -322,30 +357,40 @@ __device__ __forceinline__ void receiver_body(int rc, int P, const int64_t *__re
       s[c] = tt;
     }
   }
-  if (t < kRecThreads)
 #pragma unroll
-    for (int c = 0; c < C; ++c) part[c][t] = s[c];
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_down_sync(0xffffffffu, s[c], o);
+  __syncthreads();  // part may still be read by an earlier call's threads
+  if ((t & 31) == 0)
+#pragma unroll
+    for (int c = 0; c < C; ++c) part[c][t >> 5] = s[c];
   __syncthreads();
-  for (int o = kRecThreads / 2; o > 0; o >>= 1) {
-    if (t < o)
+  if (t < C) {
+    double sum = part[t][0];
 #pragma unroll
-      for (int c = 0; c < C; ++c) part[c][t] += part[c][t + o];
-    __syncthreads();
+    for (int k = 1; k < kWarps; ++k) sum += part[t][k];
+    seis[((int64_t)rc * C + t) * cap + col] = sum;
   }
-  if (t < C) seis[((int64_t)rc * C + t) * cap + (*step % cap)] = part[t][0];
 }
 
+// What follows a step's update, in one launch: CTA b < nrec samples receiver
+// b after the step just completed (number *step - 1); the last CTA evaluates
+// the source-time functions of the step to come (SourceTerms::stf).  With
+// nrec = 0 it is the evaluation alone, before a first step.
 template <typename real, int C>
 __global__ void __launch_bounds__(kRecThreads)
-receiver_kernel(int P, const int64_t *__restrict__ elem, const double *__restrict__ lw,
-                const int32_t *__restrict__ conn, const real *__restrict__ u,
-                double *__restrict__ seis, int64_t cap, const int64_t *__restrict__ step) {
-  receiver_body<real, C>(blockIdx.x, P, elem, lw, conn, u, seis, cap, step);
+step_tail_kernel(int nrec, int P, const int64_t *__restrict__ elem, const double *__restrict__ lw,
+                 const int32_t *__restrict__ conn, const real *__restrict__ u,
+                 double *__restrict__ seis, int64_t cap, const int64_t *__restrict__ step, int nsrc,
+                 const double *__restrict__ par, double dt, double *__restrict__ stf) {
+  const int64_t n = *step;
+  if ((int)blockIdx.x < nrec) {
+    receiver_body<real, C>(blockIdx.x, P, elem, lw, conn, u, seis, cap, n - 1);
+    return;
+  }
+  source_times(nsrc, par, n, dt, stf);
 }
-
-// Advances the device step counter (one thread), after every kernel of the
-// step that reads it.
-__global__ void advance_step_kernel(int64_t *__restrict__ step) { *step += 1; }
 
 // Deterministic partial sums of x.y weighted by w (w may be null): one partial
 // per CTA, summed on the host in block order.
