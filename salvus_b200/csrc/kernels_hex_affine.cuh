@@ -3,7 +3,8 @@
 // element, so the per-point record shrinks to the folded material constants
 // (plus the connectivity, read from the [E][P] map).
 //
-// Same arithmetic as the column-threaded kernel of kernels_hex_v2.cuh
+// Orders 4 and up run the line-exchange body of kernels_hex_col.cuh on these
+// records.  Same arithmetic as the column-threaded kernel of kernels_hex_v2.cuh
 // (Elastic3D.cpp:70-118 via Hexahedra.cpp:580-632 / 689-754) with J taken
 // from the element instead of the point.  Global arrays:
 //   jac  [E][9]    invJ (row-major [x_a][xi_b]) of each element
@@ -35,17 +36,6 @@
 
 namespace salvus {
 
-// Interior-node update of the fused step: Newmark state, inverse mass, and
-// the elements that hold a source (their interior nodes are finished by the
-// source kernel, which adds the source terms).
-struct HexInteriorUpdate {
-  const float *mi;
-  float *w, *ap;  // ap: null unless this step stores a_
-  float dt;
-  int nsrc_elem;
-  const int64_t *src_elem;  // distinct source elements
-};
-
 template <int N, int EPB_, bool TI>
 struct HexAffineShape {
   using V2 = ElasticV2Shape<N, EPB_, TI>;
@@ -53,6 +43,7 @@ struct HexAffineShape {
   static constexpr int THREADS = V2::THREADS;
   static constexpr int NM = ElasticMat<TI>::kWords;
   static constexpr int US = V2::US, FS = V2::FS;
+  static constexpr bool LINES = V2::LINES;
   static constexpr size_t SMEM = V2::SMEM;
 };
 
@@ -64,6 +55,10 @@ __device__ __forceinline__ void elastic_hex_affine_body(
     const int32_t *__restrict__ conn, float *__restrict__ u, float *__restrict__ r,
     const DMatrix<float> &Dm, const HexInteriorUpdate &iu) {
   using S = HexAffineShape<N, EPB_, TI>;
+  if constexpr (S::LINES) {
+    elastic_hex_col_body<N, EPB_, float, TI, true, kFuse>(bid, E, jac, mat, conn, u, r, Dm, iu);
+    return;
+  }
   constexpr int n = S::n, n2 = S::n2, P = S::P, EPB = S::EPB, NM = S::NM;
   extern __shared__ __align__(16) float smem_af[];
   const int t = threadIdx.x;
@@ -159,18 +154,13 @@ __device__ __forceinline__ void elastic_hex_affine_body(
   }
   __syncthreads();
   if (!ok) return;
-  // interior column: both in-plane indices strictly inside the element
-  const bool icol = kFuse && i >= 1 && i <= n - 2 && j >= 1 && j <= n - 2;
   // Elements holding a source keep the unfused form for their interior
   // points (residuals written; the source kernel adds the source terms and
   // finishes those nodes).  For the others, the interior operands (w)
   // are loaded here, before the divergence, so that their latency overlaps
   // it (after the stores below the compiler could not reorder them: the
   // pointers may alias as far as it knows).
-  bool fuse_here = icol;
-  if constexpr (kFuse) {
-    for (int s = 0; s < iu.nsrc_elem && fuse_here; ++s) fuse_here = __ldg(iu.src_elem + s) != e;
-  }
+  const bool fuse_here = kFuse && fuse_column<n>(i, j, e, iu);
   float wpre[n][3];
   if constexpr (kFuse) {
     if (fuse_here) {
@@ -261,8 +251,18 @@ __global__ void source_fused_hex_kernel(int P, const float *__restrict__ r, int 
   }
 }
 
+// CTAs per SM asked of the compiler for the isotropic line-exchange kernels:
+// what their registers allow anyway, but it schedules for it (order 4, 64^3:
+// 373 -> 367 us; order 5, 18^3: 20.5 -> 18.9 us).
 template <int N, int EPB_, bool TI>
-__global__ void __launch_bounds__(HexAffineShape<N, EPB_, TI>::THREADS)
+constexpr int affine_min_blocks() {
+  constexpr int nominal = 128 / ((N + 1) * (N + 1)) > 0 ? 128 / ((N + 1) * (N + 1)) : 1;
+  if (TI || EPB_ != nominal) return 1;
+  return N == 4 ? 8 : N == 5 ? 7 : N == 6 ? 6 : 1;
+}
+template <int N, int EPB_, bool TI>
+__global__ void __launch_bounds__(HexAffineShape<N, EPB_, TI>::THREADS,
+                                  affine_min_blocks<N, EPB_, TI>())
 elastic_hex_affine_kernel(int64_t E, const float *__restrict__ jac, const float *__restrict__ mat,
                           const int32_t *__restrict__ conn, float *__restrict__ u,
                           float *__restrict__ r, DMatrix<float> Dm, HexInteriorUpdate iu) {

@@ -1,5 +1,6 @@
-// kernels_hex_v2.cuh -- FP32 elastic hexahedron stiffness, column threads
-// with 32-bit shared-memory planes.
+// kernels_hex_v2.cuh -- FP32 elastic hexahedron stiffness on per-point
+// records: column threads with 32-bit shared-memory planes at orders 1-3, the
+// line-exchange body of kernels_hex_col.cuh on the same records above.
 //
 // Same arithmetic as elastic_hex_stiffness_kernel (Elastic3D.cpp:70-118 via
 // Hexahedra.cpp:580-632 / 689-754).  Differences that matter on B200:
@@ -19,6 +20,7 @@
 
 #include <cstdint>
 
+#include "kernels_hex_col.cuh"
 #include "kernels_material.cuh"
 
 namespace salvus {
@@ -36,7 +38,10 @@ struct ElasticV2Shape {
   // padded per-element strides (words): u planes 3P, F planes 6P
   static constexpr int US = pad_to_mod32(3 * P, n2 % 32);
   static constexpr int FS = pad_to_mod32(6 * P, n2 % 32);
-  static constexpr size_t SMEM = sizeof(float) * (size_t)EPB * (US + FS);
+  // orders 4 and up: line exchange (kernels_hex_col.cuh)
+  static constexpr bool LINES = N >= 4;
+  static constexpr size_t SMEM = LINES ? HexColShape<N, EPB_, float>::SMEM
+                                       : sizeof(float) * (size_t)EPB * (US + FS);
 };
 
 // Records ([E][PLANES][P] float4): plane 0 = invJ 0-3, plane 1 = invJ 4-7,
@@ -49,6 +54,11 @@ __device__ __forceinline__ void elastic_hex_v2_body(int64_t bid, int64_t E,
                                                     const float *__restrict__ u,
                                                     float *__restrict__ r, const DMatrix<float> &Dm) {
   using S = ElasticV2Shape<N, EPB_, TI>;
+  if constexpr (S::LINES) {
+    elastic_hex_col_body<N, EPB_, float, TI, false, false>(
+        bid, E, nullptr, rec, nullptr, const_cast<float *>(u), r, Dm, HexInteriorUpdate{});
+    return;
+  }
   constexpr int n = S::n, n2 = S::n2, P = S::P, EPB = S::EPB;
   extern __shared__ __align__(16) float smem_v2[];
   const int t = threadIdx.x;
