@@ -575,6 +575,43 @@ static void interior_free_nodes(salvus_mesh *m) {
   m->n_gnodes = (int64_t)m->gnodes.size();
 }
 
+static bool acoustic_quads(const salvus_mesh *m) {
+  return m->shape == SALVUS_QUAD && m->physics == SALVUS_ACOUSTIC;
+}
+static Incidence incidence(const salvus_mesh *m) {
+  return {m->d_inc_head.as<int2>(), m->d_inc_rest.as<int32_t>()};
+}
+// Two nodes per thread (gather_pair_kernel): acoustic quadrilaterals with six
+// CTAs of nodes per SM (227 k nodes) or more; fewer leave SMs without enough
+// warps to hide the chain (40 k-116 k nodes: 5.3-5.5 us a step with one node
+// per thread, 5.4-6.0 with two; 361 k: 8.1 against 7.2-7.6).  Orders 1 and 2
+// are mostly vertices, whose lists take the longer way (500^2 order 1: 8.3
+// against 9.1 us).
+static bool gather_pairs(const salvus_mesh *m, int64_t nodes) {
+  return acoustic_quads(m) && m->order >= 3 && nodes >= 6 * (int64_t)kPairTile * m->sm_count;
+}
+
+static int upload_heads(salvus_mesh *m) {
+  std::vector<int2> head((size_t)m->G);
+  std::vector<int32_t> rest(1, 0);
+  for (int64_t g = 0; g < m->G; ++g) {
+    const int32_t q0 = m->inc_off[(size_t)g], n = m->inc_off[(size_t)g + 1] - q0;
+    const int32_t *q = m->inc_idx.data() + q0;
+    head[(size_t)g] = n > 2 ? int2{(int32_t)rest.size(), -n} : int2{q[0], n == 2 ? q[1] : -1};
+    if (n > 2) rest.insert(rest.end(), q, q + n);
+  }
+  int rc;
+  if ((rc = m->d_inc_head.alloc(sizeof(int2) * head.size())) ||
+      (rc = m->d_inc_rest.alloc(sizeof(int32_t) * rest.size())))
+    return rc;
+  SALVUS_CUDA(cudaMemcpyAsync(m->d_inc_head.ptr, head.data(), sizeof(int2) * head.size(),
+                              cudaMemcpyHostToDevice, m->stream));
+  SALVUS_CUDA(cudaMemcpyAsync(m->d_inc_rest.ptr, rest.data(), sizeof(int32_t) * rest.size(),
+                              cudaMemcpyHostToDevice, m->stream));
+  SALVUS_CUDA(cudaStreamSynchronize(m->stream));  // the vectors end here
+  return SALVUS_OK;
+}
+
 static int mesh_setup_device(salvus_mesh *m) {
   int rc;
   SALVUS_CUDA(cudaSetDevice(m->device));
@@ -621,6 +658,7 @@ static int mesh_setup_device(salvus_mesh *m) {
     }
     SALVUS_CUDA(cudaStreamSynchronize(m->stream));
   }
+  if (acoustic_quads(m) && (rc = upload_heads(m))) return rc;
   DeviceBuffer mass_local;
   if ((rc = mass_local.alloc(sizeof(double) * EP))) return rc;
   if (m->affine) {
@@ -918,10 +956,6 @@ static bool hex_interior_fusion(const salvus_problem *p) {
   return p->hex_form == 1;
 }
 
-// 128-thread CTAs of the step's node gather: measured against 64 / 256 / 512
-// on the benchmark meshes, 1 % (hexahedra) to 5 % (tetrahedra) faster than 256
-constexpr int kGatherThreads = 128;
-
 template <bool TI>
 static int launch_fused_interior(salvus_problem *p, const HexInteriorUpdate &iu) {
   const salvus_mesh *m = p->mesh;
@@ -1009,11 +1043,17 @@ static int step_fused_t(salvus_problem *p, bool store_a) {
   if ((rc = launch_coupling<real>(p))) return rc;
   {
     ProfScope ps(p, K_UPDATE);
-    gather_kernel<real, C, 0><<<blocks_for(m->G, kGatherThreads), kGatherThreads, 0, p->stream>>>(
-        m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<real>(p->d_r),
-        inv_mass<real>(p), F<real>(p->d_u), F<real>(p->d_v),
-        store_a || m->physics == SALVUS_COUPLED2D ? F<real>(p->d_ap) : nullptr, nullptr,
-        (real)p->dt, source_terms(p), p->d_step.as<int64_t>());
+    if (C == 1 && gather_pairs(m, m->G))
+      gather_pair_kernel<real><<<blocks_for(m->G, kPairTile), kGatherThreads, 0, p->stream>>>(
+          m->G, incidence(m), F<real>(p->d_r), inv_mass<real>(p), F<real>(p->d_u), F<real>(p->d_v),
+          store_a ? F<real>(p->d_ap) : nullptr, (real)p->dt, source_terms(p),
+          p->d_step.as<int64_t>());
+    else
+      gather_kernel<real, C, 0><<<blocks_for(m->G, kGatherThreads), kGatherThreads, 0, p->stream>>>(
+          m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<real>(p->d_r),
+          inv_mass<real>(p), F<real>(p->d_u), F<real>(p->d_v),
+          store_a || m->physics == SALVUS_COUPLED2D ? F<real>(p->d_ap) : nullptr, nullptr,
+          (real)p->dt, source_terms(p), p->d_step.as<int64_t>());
     g_launches++;
     if ((rc = check_launch("gather update"))) return rc;
   }
@@ -1099,7 +1139,7 @@ static void launch_bg(const salvus_problem *p, cudaStream_t st, bool fuse, int64
   const int64_t n = fuse ? m->n_gnodes : m->G;
   dim3 grid((unsigned)((n + NPB * NPT - 1) / (NPB * NPT)), (unsigned)(p->shots_pad / SC));
   batched_gather_update_kernel<SC, NPB, NPT><<<grid, SC * NPB, 0, st>>>(
-      n, p->shots_pad, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(),
+      n, p->shots_pad, incidence(m),
       F<float>(p->d_r), m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v), (float)p->dt,
       fuse ? m->d_gnodes.as<int32_t>() : nullptr, step);
 }
@@ -1417,8 +1457,8 @@ static int launch_finite_check(salvus_problem *p) {
   return check_launch("finite check");
 }
 
-// Hexahedron autotuner (FP32 elastic meshes of parallelepipeds, one shot):
-// times the plain step (stiffness, node gather/update) with CTAs of 128 /
+// Hexahedron autotuner (FP32 elastic meshes of parallelepipeds of orders 1-3,
+// one shot): times the plain step (stiffness, node gather/update) with CTAs of 128 /
 // (N+1)^2 elements and with twice as many, on zeroed scratch copies of u and
 // w, and keeps the faster.  Both give bitwise the same wavefield (the same
 // arithmetic per element and per node, in the same order), so the choice
@@ -1453,6 +1493,14 @@ static int tune_hex(salvus_problem *p) {
       m->hex_wide = b;
       return SALVUS_OK;
     }
+  }
+  // line-exchange kernels (orders 4 and up): the narrow CTA was the faster one
+  // on every mesh measured (64^3 order 4: 0.377 against 0.434 ms), and on
+  // small ones a few timed launches picked the slower (16^3: 15.4 against 13.9
+  // us a step)
+  if (m->order >= 4) {
+    p->hex_form = 0;
+    return SALVUS_OK;
   }
   // problems are prepared on several threads (the job server)
   static std::mutex cache_mu;
@@ -1606,6 +1654,7 @@ struct salvus_group {
   std::vector<int32_t> owner;
   salvus::DeviceBuffer d_owner;
   int64_t n_stiff = 0, n_gather = 0, n_rec = 0;
+  bool pairs = false;  // two nodes per thread in the gather
   // persistent single-launch step: work-item queue
   std::vector<salvus::GroupCounts> counts;
   std::vector<salvus::GroupWork> work;
@@ -1649,6 +1698,7 @@ static int group_fill(salvus_group *g) {
     s.conn = m->d_conn.as<int32_t>();
     s.inc_off = m->d_inc_off.as<int32_t>();
     s.inc_idx = m->d_inc_idx.as<int32_t>();
+    s.inc = incidence(m);
     s.mi = m->d_mi32.as<float>();
     s.E = m->E;
     s.G = m->G;
@@ -1672,9 +1722,12 @@ static int group_fill(salvus_group *g) {
     s.b_gather = bg;
     s.b_rec = br;
     bs += group_stiff_blocks(m);
-    bg += (m->G + 255) / 256;
+    bg += (m->G + 255) / 256;  // 256 nodes per CTA in both forms (kPairTile)
     br += s.nrec + (s.nsrc > 0 ? 1 : 0);
   }
+  int64_t nodes = 0;
+  for (auto *p : g->members) nodes += p->mesh->G;
+  g->pairs = gather_pairs(g->m0, nodes);
   g->n_stiff = bs;
   g->n_gather = bg;
   g->n_rec = br;
@@ -1893,7 +1946,9 @@ static int group_step(salvus_group *g, bool store_a) {
   int rc;
   const int32_t *own = g->d_owner.as<int32_t>();
   if ((rc = group_stiffness(g->m0, slots, own, g->n_stiff, g->stream))) return rc;
-  if (g->c == 1) group_gather_update<1><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff, store_a);
+  if (g->pairs)
+    group_gather_pairs<<<(unsigned)g->n_gather, kGatherThreads, 0, g->stream>>>(slots, own + g->n_stiff, store_a);
+  else if (g->c == 1) group_gather_update<1><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff, store_a);
   else group_gather_update<3><<<(unsigned)g->n_gather, 256, 0, g->stream>>>(slots, own + g->n_stiff, store_a);
   if (g->n_rec > 0) {
     const int32_t *own_rec = own + g->n_stiff + g->n_gather;

@@ -132,6 +132,7 @@ struct salvus_mesh {
   int64_t n_cpl = 0, n_cpl_fluid = 0;  // fluid points first
   // device
   salvus::DeviceBuffer d_conn, d_inc_off, d_inc_idx, d_vtx, d_par;
+  salvus::DeviceBuffer d_inc_head, d_inc_rest;  // acoustic quadrilaterals (Incidence)
   salvus::DeviceBuffer d_mi64, d_mi32;
   salvus::DeviceBuffer d_rec32, d_rec64;  // stiffness records per precision
   // elastic hexahedra that are all parallelepipeds: d_rec32 holds material

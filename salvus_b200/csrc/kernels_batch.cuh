@@ -171,15 +171,14 @@ __global__ void batched_source_kernel(int S, int P, const int32_t *__restrict__ 
 
 // Node gather + inverse mass + half-step-velocity update, thread = (NPT
 // consecutive nodes, shot).  CTA = NPB node groups x SC shots.  The NPT
-// nodes' dependent load chains (offsets -> incidence -> residual) are issued
+// nodes' dependent load chains (incidence -> residual) are issued
 // side by side so that more bytes are in flight per thread; the per-node
 // arithmetic and summation order do not depend on NPT.
 // nodes != nullptr: thread slot t handles node nodes[t] (the edge nodes of
 // the fused form), G is then the list's length.
 template <int SC, int NPB, int NPT>
 __global__ void __launch_bounds__(SC *NPB)
-batched_gather_update_kernel(int64_t G, int S, const int32_t *__restrict__ off,
-                             const int32_t *__restrict__ idx, const float *__restrict__ r,
+batched_gather_update_kernel(int64_t G, int S, Incidence inc, const float *__restrict__ r,
                              const float *__restrict__ mi, float *__restrict__ u,
                              float *__restrict__ w, float dt,
                              const int32_t *__restrict__ nodes, int64_t *__restrict__ step) {
@@ -190,7 +189,8 @@ batched_gather_update_kernel(int64_t G, int S, const int32_t *__restrict__ off,
   if (g0 >= G || s >= S) return;
   constexpr int kFast = 4;  // quadrilateral valence bound
   float uo[NPT], wo[NPT], m[NPT];
-  int32_t q0[NPT], cnt[NPT];
+  int2 h[NPT];
+  int32_t cnt[NPT];
   int64_t gk[NPT];
 #pragma unroll
   for (int k = 0; k < NPT; ++k) {
@@ -201,15 +201,16 @@ batched_gather_update_kernel(int64_t G, int S, const int32_t *__restrict__ off,
     uo[k] = live ? u[i] : 0.f;
     wo[k] = live ? w[i] : 0.f;
     m[k] = live ? __ldg(mi + g) : 0.f;
-    q0[k] = live ? __ldg(off + g) : 0;
-    cnt[k] = live ? __ldg(off + g + 1) - q0[k] : 0;
+    h[k] = live ? __ldg(inc.head + g) : int2{0, 0};
+    cnt[k] = !live ? 0 : h[k].y >= -1 ? 1 + (h[k].y >= 0) : -h[k].y;
   }
   // all incidence indices first, then all residual loads in flight at once
   int32_t ep[NPT][kFast];
 #pragma unroll
   for (int k = 0; k < NPT; ++k)
 #pragma unroll
-    for (int q = 0; q < kFast; ++q) ep[k][q] = q < cnt[k] ? __ldg(idx + q0[k] + q) : 0;
+    for (int q = 0; q < kFast; ++q)
+      ep[k][q] = q >= cnt[k] ? 0 : cnt[k] > 2 ? __ldg(inc.rest + h[k].x + q) : q == 0 ? h[k].x : h[k].y;
   float rv[NPT][kFast];
 #pragma unroll
   for (int k = 0; k < NPT; ++k)
@@ -227,8 +228,8 @@ batched_gather_update_kernel(int64_t G, int S, const int32_t *__restrict__ off,
       for (int q = 0; q < kFast; ++q)
         if (q < cnt[k]) acc += rv[k][q];
     } else {
-      for (int32_t q = q0[k]; q < q0[k] + cnt[k]; ++q)
-        acc += __ldg(r + (int64_t)__ldg(idx + q) * S + s);
+      for (int32_t q = h[k].x; q < h[k].x + cnt[k]; ++q)
+        acc += __ldg(r + (int64_t)__ldg(inc.rest + q) * S + s);
     }
     float wn = wo[k], un = uo[k];
     half_step_update(acc, m[k], dt, wn, un);

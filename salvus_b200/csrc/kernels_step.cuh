@@ -217,6 +217,124 @@ __global__ void gather_kernel(int64_t G, const int32_t *__restrict__ off,
                              w, ap, a, dt, src);
 }
 
+// Incidence of quadrilateral meshes, as the kernels below and the batched
+// gather read it: one pair per node holds the whole list of element points
+// e*P + p where it has one entry (x, -1) or two (x, y) -- 94 % of the nodes of
+// an order-4 mesh -- so that the residual loads depend on one load, not on an
+// offset and then an index; longer lists (vertices) are rest[x, x - y) with
+// y = -length.
+struct Incidence {
+  const int2 *head;
+  const int32_t *rest;
+};
+
+// Gather and update (mode 0 of gather_body, the same arithmetic) of two
+// adjacent nodes of a 1-component quadrilateral mesh, g even: every stream is
+// one 64- or 128-bit access for both nodes.  Half the threads and two thirds
+// of the instructions of one node per thread; what remains is DRAM traffic
+// and the chain head -> residual.  Per step, order 4: 400^2 41.2 -> 37.4 us,
+// 700^2 121 -> 112, 16 grouped meshes of 10^2-90^2 22.2 -> 18.3; FP64 150^2
+// order 7 29.6 -> 25.1 (B200).  Other element classes keep one node per
+// thread: on triangles (six-element vertices) 19.5 us became 21.1, and on
+// 3-component fields pairs or heads changed a step by -1 to +8 %.
+template <typename real, bool kInKernelR = false>
+__device__ __forceinline__ void gather_pair_body(int64_t g, int64_t G, const Incidence &inc,
+                                                 const real *__restrict__ r,
+                                                 const real *__restrict__ mi, real *__restrict__ u,
+                                                 real *__restrict__ w, real *__restrict__ ap,
+                                                 real dt, const SourceTerms &src) {
+  if (g >= G) return;
+  struct alignas(2 * sizeof(real)) Pair {
+    real v[2];
+  };
+  const bool two = g + 1 < G;
+  int2 h[2];
+  Pair m, uo, wo;
+  if (two) {
+    const int4 hh = *reinterpret_cast<const int4 *>(inc.head + g);
+    h[0] = {hh.x, hh.y};
+    h[1] = {hh.z, hh.w};
+    m = *reinterpret_cast<const Pair *>(mi + g);
+    uo = *reinterpret_cast<const Pair *>(u + g);
+    wo = *reinterpret_cast<const Pair *>(w + g);
+  } else {
+    h[0] = inc.head[g];
+    h[1] = {h[0].x, -1};
+    m.v[0] = m.v[1] = mi[g];
+    uo.v[0] = uo.v[1] = u[g];
+    wo.v[0] = wo.v[1] = w[g];
+  }
+  const int32_t src_at = src.tile ? src.tile[g / kSrcTile] : -1;
+  auto load = [&](int32_t ep) -> real { return kInKernelR ? __ldca(r + ep) : r[ep]; };
+  real acc[2], second[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    acc[q] = h[q].y >= -1 ? load(h[q].x) : real(0);
+    second[q] = h[q].y >= 0 ? load(h[q].y) : real(0);
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    acc[q] = add_rn(real(0), acc[q]);  // the general gather's first addition
+    if (h[q].y >= 0) {
+      acc[q] += second[q];
+    } else if (h[q].y < -1) {
+      constexpr int kBatch = 4;  // the usual valence of a quadrilateral vertex
+      const int32_t q1 = h[q].x - h[q].y;
+      for (int32_t qb = h[q].x; qb < q1; qb += kBatch) {
+        int32_t ep[kBatch];
+        real rv[kBatch];
+#pragma unroll
+        for (int z = 0; z < kBatch; ++z) ep[z] = qb + z < q1 ? inc.rest[qb + z] : 0;
+#pragma unroll
+        for (int z = 0; z < kBatch; ++z) rv[z] = qb + z < q1 ? load(ep[z]) : real(0);
+#pragma unroll
+        for (int z = 0; z < kBatch; ++z)
+          if (qb + z < q1) acc[q] += rv[z];
+      }
+    }
+  }
+  if (src_at >= 0) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      real aq[1] = {acc[q]};
+      if (q == 0 || two)
+        add_sources<real, 1, kInKernelR>(src.node[src_at + (g + q) % kSrcTile], src, aq);
+      acc[q] = aq[0];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    acc[q] = mul_rn(acc[q], m.v[q]);
+    newmark_point<real>(acc[q], wo.v[q], uo.v[q], dt);
+  }
+  if (two) {
+    *reinterpret_cast<Pair *>(u + g) = uo;
+    *reinterpret_cast<Pair *>(w + g) = wo;
+    if (ap) *reinterpret_cast<Pair *>(ap + g) = Pair{acc[0], acc[1]};
+  } else {
+    u[g] = uo.v[0];
+    w[g] = wo.v[0];
+    if (ap) ap[g] = acc[0];
+  }
+}
+
+// 128-thread CTAs of the step's node gathers: measured against 64 / 256 / 512
+// on the benchmark meshes, 1 % (hexahedra) to 5 % (tetrahedra) faster than 256
+constexpr int kGatherThreads = 128;
+constexpr int kPairTile = 2 * kGatherThreads;  // nodes per CTA
+
+// CTAs per SM asked of the compiler: FP32 12 (10: 38.7 us on 400^2, 118 on
+// 700^2), FP64 10 (12: 28.8 on 150^2 order 7).
+template <typename real>
+__global__ void __launch_bounds__(kGatherThreads, sizeof(real) == 4 ? 12 : 10)
+gather_pair_kernel(int64_t G, Incidence inc, const real *__restrict__ r,
+                   const real *__restrict__ mi, real *__restrict__ u, real *__restrict__ w,
+                   real *__restrict__ ap, real dt, SourceTerms src, int64_t *__restrict__ step) {
+  const int64_t t = (int64_t)blockIdx.x * kGatherThreads + threadIdx.x;
+  if (t == 0) *step += 1;  // nothing else of the launch reads it
+  gather_pair_body<real>(2 * t, G, inc, r, mi, u, w, ap, dt, src);
+}
+
 // The gather / update over a list of nodes (the shared nodes of a fused
 // hexahedron step, whose interior nodes the stiffness kernel advanced).
 template <typename real, int C, int MODE>
