@@ -111,9 +111,9 @@ static int launch_acoustic(const salvus_mesh *m, const real *rec, const real *u,
 }
 
 // FP32 elastic hexahedra: the column-threaded kernel with 32-bit shared
-// planes and 128-thread CTAs (whole warps: 5 order-4 elements, 6 CTAs per
-// SM) by default; SALVUS_HEX_KERNEL=classic selects the register / shared-
-// memory kernel that also serves FP64 (read at every launch).
+// planes and 128-thread CTAs (whole warps: 5 order-4 elements) by default;
+// SALVUS_HEX_KERNEL=classic selects the register / shared-memory kernel that
+// also serves FP64 general hexahedra of order 3 (read at every launch).
 static bool hex_classic() {
   const char *s = std::getenv("SALVUS_HEX_KERNEL");
   return s && std::strcmp(s, "classic") == 0;
@@ -181,6 +181,24 @@ static int launch_elastic_affine(const salvus_mesh *m, const float *mat, float *
                      : launch_elastic_affine_epb<N, EPB, TI, kFuse>(m, mat, u, r, st, iu);
 }
 
+template <int N, bool TI, bool kAffine>
+static int launch_elastic_col64(const salvus_mesh *m, const double *rec, const double *u, double *r,
+                                cudaStream_t st) {
+  constexpr int EPB = HexCol64<N, TI, kAffine>::EPB;
+  using T = HexColShape<N, EPB, double>;
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(elastic_hex_col64_kernel<N, TI, kAffine>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
+    attr = true;
+  }
+  elastic_hex_col64_kernel<N, TI, kAffine><<<blocks_for(m->E, EPB), T::THREADS, T::SMEM, st>>>(
+      m->E, m->d_jac64.as<double>(), rec, m->d_conn.as<int32_t>(), const_cast<double *>(u), r,
+      dmatrix<double>(m->basis));
+  g_launches++;
+  return check_launch("elastic stiffness");
+}
+
 template <int N, typename real>
 static int launch_elastic(const salvus_mesh *m, const real *rec, const real *u, real *r,
                           cudaStream_t st) {
@@ -193,9 +211,17 @@ static int launch_elastic(const salvus_mesh *m, const real *rec, const real *u, 
     if (!hex_classic())
       return m->ti ? launch_elastic_v2<N, true>(m, rec, u, r, st)
                    : launch_elastic_v2<N, false>(m, rec, u, r, st);
+  } else {
+    if (m->affine64)
+      return m->ti ? launch_elastic_col64<N, true, true>(m, rec, u, r, st)
+                   : launch_elastic_col64<N, false, true>(m, rec, u, r, st);
+    if constexpr (HexCol64<N, false, false>::kUse)
+      return m->ti ? launch_elastic_col64<N, true, false>(m, rec, u, r, st)
+                   : launch_elastic_col64<N, false, false>(m, rec, u, r, st);
   }
-  return m->ti ? launch_elastic_classic<N, real, true>(m, rec, u, r, st)
-               : launch_elastic_classic<N, real, false>(m, rec, u, r, st);
+  if constexpr (sizeof(real) == 4 || !HexCol64<N, false, false>::kUse)
+    return m->ti ? launch_elastic_classic<N, real, true>(m, rec, u, r, st)
+                 : launch_elastic_classic<N, real, false>(m, rec, u, r, st);
 }
 
 // Quadrilateral stiffness: column-threaded kernels (kernels_quad_col.cuh) by
@@ -672,10 +698,19 @@ static int mesh_setup_device(salvus_mesh *m) {
       gll.xi[i] = m->basis.xi[i];
       gll.w[i] = m->basis.w[i];
     }
-    affine_hex_records_kernel<<<blocks_for(EP, 128), 128, 0, m->stream>>>(
+    affine_hex_records_kernel<float><<<blocks_for(EP, 128), 128, 0, m->stream>>>(
         m->E, m->n, m->P, m->ti, m->d_vtx.as<double>(), m->d_par.as<double>(), gll,
         m->d_rec32.as<float>(), m->d_jac32.as<float>(), mass_local.as<double>());
     g_launches++;
+    if (m->affine64 && !m->fp32_only) {
+      if ((rc = m->d_rec64.alloc(sizeof(double) * (size_t)nm * EP)) ||
+          (rc = m->d_jac64.alloc(sizeof(double) * 9 * (size_t)m->E)))
+        return rc;
+      affine_hex_records_kernel<double><<<blocks_for(EP, 128), 128, 0, m->stream>>>(
+          m->E, m->n, m->P, m->ti, m->d_vtx.as<double>(), m->d_par.as<double>(), gll,
+          m->d_rec64.as<double>(), m->d_jac64.as<double>(), mass_local.as<double>());
+      g_launches++;
+    }
     if ((rc = check_launch("affine records"))) return rc;
   } else if ((rc = build_records<float, true>(m, m->d_rec32, mass_local))) {
     return rc;
@@ -687,7 +722,9 @@ static int mesh_setup_device(salvus_mesh *m) {
                                 cudaMemcpyHostToDevice, m->stream));
     SALVUS_CUDA(cudaStreamSynchronize(m->stream));
   }
-  if (!m->fp32_only && (rc = build_records<double, false>(m, m->d_rec64, mass_local))) return rc;
+  if (!m->fp32_only && !m->affine64 &&
+      (rc = build_records<double, false>(m, m->d_rec64, mass_local)))
+    return rc;
   mass_gather_kernel<<<blocks_for(m->G, 256), 256, 0, m->stream>>>(
       m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), mass_local.as<double>(),
       m->d_mi64.as<double>(), m->d_mi32.as<float>());
@@ -2095,23 +2132,30 @@ int salvus_mesh_create(const salvus_mesh_desc *d, int device, salvus_mesh **out)
   if (m->shape == SALVUS_HEX && m->physics == SALVUS_ELASTIC3D &&
       !(d->reserved & SALVUS_MESH_PER_POINT_GEOMETRY)) {
     // every element a parallelepiped: the inverse Jacobian at the eight
-    // corners equals the one at the centre (to 1e-12 relative)
-    bool affine = true;
+    // corners equals the one at the centre (to 1e-12 relative; FP64 takes the
+    // one Jacobian only where they agree to the rounding of the coordinates,
+    // 16 eps |x| / h relative)
+    bool affine = true, affine64 = true;
     for (int64_t e = 0; e < m->E && affine; ++e) {
       const double *v = m->vtx.data() + e * 24;
       double c0[3] = {0, 0, 0}, det0, J0[9];
       p1_jacobian(m->shape, v, c0, &det0, J0);
-      double scale = 0;
+      double scale = 0, far = 0;
       for (int a = 0; a < 9; ++a) scale = std::max(scale, std::fabs(J0[a]));
+      for (int a = 0; a < 24; ++a) far = std::max(far, std::fabs(v[a]));
+      const double tol64 = 16.0 * 2.220446049250313e-16 * far * scale;
       for (int q = 0; q < 8 && affine; ++q) {
         double ref[3], det, J[9];
         for (int a = 0; a < 3; ++a) ref[a] = ((q >> a) & 1) ? 1.0 : -1.0;
         p1_jacobian(m->shape, v, ref, &det, J);
-        for (int a = 0; a < 9; ++a)
+        for (int a = 0; a < 9; ++a) {
           if (std::fabs(J[a] - J0[a]) > 1e-12 * scale) affine = false;
+          if (std::fabs(J[a] - J0[a]) > tol64 * scale) affine64 = false;
+        }
       }
     }
     m->affine = affine;
+    m->affine64 = affine && affine64;
   }
   if ((rc = flatten_mesh(m.get(), d->cells, d->n_vertices))) return rc;
   if (m->physics == SALVUS_COUPLED2D && (rc = setup_coupled(m.get(), d->cells))) return rc;

@@ -139,10 +139,13 @@ struct salvus_mesh {
   // planes [NM][E*P], d_jac32 the per-element invJ [E][9]; d_gnodes lists
   // the nodes that are not interior to an element (fused steps' gather)
   bool affine = false;
+  // the same for FP64 (d_rec64, d_jac64): the Jacobians agree to the rounding
+  // of the vertex coordinates
+  bool affine64 = false;
   // parallelepiped hexahedron kernels: CTAs of 128 / (N+1)^2 elements (0) or
   // twice that (1), set by the hexahedron autotuner
   int hex_wide = 0;
-  salvus::DeviceBuffer d_jac32, d_gnodes;
+  salvus::DeviceBuffer d_jac32, d_jac64, d_gnodes;
   std::vector<int32_t> gnodes;  // host copy of d_gnodes
   int64_t n_gnodes = 0;
   salvus::DeviceBuffer d_sd32, d_sd64;    // simplex derivative tables [dim][P][P]

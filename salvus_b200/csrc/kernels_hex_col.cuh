@@ -1,5 +1,5 @@
-// kernels_hex_col.cuh -- elastic hexahedron stiffness of orders 4 and up, r_e
-// = -K_e u_e, by column threads and line exchange (Elastic3D.cpp:70-118 via
+// kernels_hex_col.cuh -- elastic hexahedron stiffness of orders 4 and up (FP64:
+// of every order, see HexCol64), r_e = -K_e u_e, by column threads and line exchange (Elastic3D.cpp:70-118 via
 // Hexahedra.cpp:580-632 / 689-754).
 //
 // What bounds the kernel is the shared-memory pipe: a shared load delivers 32
@@ -311,6 +311,35 @@ __device__ __forceinline__ void elastic_hex_col_body(
       for (int c = 0; c < 3; ++c) r[(e * P + ij + n2 * k) * 3 + c] = out[c];
     }
   }
+}
+
+// FP64 kernels.  The FP64 column kernel (elastic_hex_stiffness_kernel) reads
+// 88-byte records point by point; on meshes of parallelepipeds this body reads
+// 16 bytes of material per point and one Jacobian per element instead, and
+// runs at every order.  Elements per CTA and CTAs per SM by measurement (B200,
+// us, FP64 column kernel -> here): 22^3 order 4 57.4 -> 33.2 (4 CTAs asked;
+// 35.3 without), 18^3 order 5 83.7 -> 37.2, 12^3 order 6 29.1 -> 20.8, 28^3
+// order 3 45.2 -> 31.0 (64-thread CTAs; 33.0 with 128), 36^3 order 2 53.6 ->
+// 33.1, 50^3 order 1 43.2 -> 24.9.  General hexahedra keep their records:
+// order 4 51.6, order 5 53.8 (4 CTAs asked; 59.7), order 6 24.8 (one element
+// per CTA), order 2 49.3, order 1 39.2; order 3 stays on the column kernel
+// (45.2 against 49.6).
+template <int N, bool TI, bool kAffine>
+struct HexCol64 {
+  static constexpr int n2 = (N + 1) * (N + 1);
+  static constexpr int kThreads = N >= 4 && !(N == 6 && !kAffine) ? 128 : 64;
+  static constexpr int EPB = kThreads / n2 > 0 ? kThreads / n2 : 1;
+  static constexpr int CTAS = !TI && N == (kAffine ? 4 : 5) ? 4 : 1;
+  static constexpr bool kUse = kAffine || N != 3;
+};
+template <int N, bool TI, bool kAffine>
+__global__ void __launch_bounds__(HexColShape<N, HexCol64<N, TI, kAffine>::EPB, double>::THREADS,
+                                  HexCol64<N, TI, kAffine>::CTAS)
+elastic_hex_col64_kernel(int64_t E, const double *__restrict__ jac, const double *__restrict__ rec,
+                         const int32_t *__restrict__ conn, double *__restrict__ u,
+                         double *__restrict__ r, DMatrix<double> Dm) {
+  elastic_hex_col_body<N, HexCol64<N, TI, kAffine>::EPB, double, TI, kAffine, false>(
+      blockIdx.x, E, jac, rec, conn, u, r, Dm, HexInteriorUpdate{});
 }
 
 }  // namespace salvus

@@ -238,16 +238,17 @@ __global__ void geometry_kernel(int64_t E, int dim, int n, int P, int physics, i
   }
 }
 
-// FP32 records of elastic hexahedra that are all parallelepipeds
+// Records of elastic hexahedra that are all parallelepipeds
 // (kernels_hex_affine.cuh): one thread per element point writes the folded
 // material planes mat[m][e*P + p] (w detJ at the point times the constants
 // of the P1-interpolated parameters, as geometry_kernel) and the
 // element-local mass; point 0 of each element also writes invJ at the
 // element centre to jac[e][9] (constant over an affine element).
+template <typename real>
 __global__ void affine_hex_records_kernel(int64_t E, int n, int P, bool ti,
                                           const double *__restrict__ vtx,
                                           const double *__restrict__ par, GllTable gll,
-                                          float *__restrict__ mat, float *__restrict__ jac,
+                                          real *__restrict__ mat, real *__restrict__ jac,
                                           double *__restrict__ mass_local) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= E * P) return;
@@ -272,13 +273,13 @@ __global__ void affine_hex_records_kernel(int64_t E, int n, int P, bool ti,
   const int nm = ti ? 5 : 2;
   if (ti) elastic_constants_ti(pv, mc);
   else elastic_constants_iso(pv[0], pv[1], pv[2], mc);
-  for (int q = 0; q < nm; ++q) mat[(int64_t)q * E * P + tid] = (float)(wd * mc[q]);
+  for (int q = 0; q < nm; ++q) mat[(int64_t)q * E * P + tid] = (real)(wd * mc[q]);
   mass_local[tid] = wd * pv[0];
   if (p == 0) {
     const double c0[3] = {0.0, 0.0, 0.0};
     double d0, J0[9];
     p1_jac_dev(3, v, c0, &d0, J0);
-    for (int a = 0; a < 9; ++a) jac[e * 9 + a] = (float)J0[a];
+    for (int a = 0; a < 9; ++a) jac[e * 9 + a] = (real)J0[a];
   }
 }
 
