@@ -1104,9 +1104,9 @@ struct BatchCfg {
 };
 static const BatchCfg kStiffCfg[] = {{32, 1, 1}, {32, 2, 1}, {32, 4, 1}, {64, 1, 1},
                                      {64, 2, 1}, {128, 1, 1}, {128, 2, 1}, {256, 1, 1}};
-static const BatchCfg kGatherCfg[] = {{32, 4, 1},  {32, 8, 1}, {64, 2, 1}, {64, 4, 1},
-                                      {128, 1, 1}, {128, 2, 1}, {256, 1, 1}, {32, 4, 2},
-                                      {64, 2, 2},  {128, 1, 2}, {128, 1, 4}, {256, 1, 2}};
+static const BatchCfg kGatherCfg[] = {{32, 16, 1}, {32, 32, 1}, {64, 8, 1}, {64, 16, 1},
+                                      {128, 4, 1}, {128, 8, 1}, {256, 2, 1}, {256, 4, 1},
+                                      {32, 16, 2}, {64, 8, 2},  {128, 4, 2}, {256, 2, 2}};
 constexpr int kNumStiffCfg = sizeof(kStiffCfg) / sizeof(kStiffCfg[0]);
 constexpr int kNumGatherCfg = sizeof(kGatherCfg) / sizeof(kGatherCfg[0]);
 
@@ -1175,7 +1175,7 @@ static void launch_bg(const salvus_problem *p, cudaStream_t st, bool fuse, int64
   const salvus_mesh *m = p->mesh;
   const int64_t n = fuse ? m->n_gnodes : m->G;
   dim3 grid((unsigned)((n + NPB * NPT - 1) / (NPB * NPT)), (unsigned)(p->shots_pad / SC));
-  batched_gather_update_kernel<SC, NPB, NPT><<<grid, SC * NPB, 0, st>>>(
+  batched_gather_update_kernel<SC, NPB, NPT><<<grid, SC / 4 * NPB, 0, st>>>(
       n, p->shots_pad, incidence(m),
       F<float>(p->d_r), m->d_mi32.as<float>(), F<float>(p->d_u), F<float>(p->d_v), (float)p->dt,
       fuse ? m->d_gnodes.as<int32_t>() : nullptr, step);
@@ -1185,18 +1185,18 @@ static void launch_bg(const salvus_problem *p, cudaStream_t st, bool fuse, int64
 static int batched_gather(const salvus_problem *p, int cfg, cudaStream_t st, bool fuse,
                           int64_t *step) {
   switch (cfg) {
-    case 0: launch_bg<32, 4>(p, st, fuse, step); break;
-    case 1: launch_bg<32, 8>(p, st, fuse, step); break;
-    case 2: launch_bg<64, 2>(p, st, fuse, step); break;
-    case 3: launch_bg<64, 4>(p, st, fuse, step); break;
-    case 4: launch_bg<128, 1>(p, st, fuse, step); break;
-    case 5: launch_bg<128, 2>(p, st, fuse, step); break;
-    case 6: launch_bg<256, 1>(p, st, fuse, step); break;
-    case 7: launch_bg<32, 4, 2>(p, st, fuse, step); break;
-    case 8: launch_bg<64, 2, 2>(p, st, fuse, step); break;
-    case 9: launch_bg<128, 1, 2>(p, st, fuse, step); break;
-    case 10: launch_bg<128, 1, 4>(p, st, fuse, step); break;
-    case 11: launch_bg<256, 1, 2>(p, st, fuse, step); break;
+    case 0: launch_bg<32, 16>(p, st, fuse, step); break;
+    case 1: launch_bg<32, 32>(p, st, fuse, step); break;
+    case 2: launch_bg<64, 8>(p, st, fuse, step); break;
+    case 3: launch_bg<64, 16>(p, st, fuse, step); break;
+    case 4: launch_bg<128, 4>(p, st, fuse, step); break;
+    case 5: launch_bg<128, 8>(p, st, fuse, step); break;
+    case 6: launch_bg<256, 2>(p, st, fuse, step); break;
+    case 7: launch_bg<256, 4>(p, st, fuse, step); break;
+    case 8: launch_bg<32, 16, 2>(p, st, fuse, step); break;
+    case 9: launch_bg<64, 8, 2>(p, st, fuse, step); break;
+    case 10: launch_bg<128, 4, 2>(p, st, fuse, step); break;
+    case 11: launch_bg<256, 2, 2>(p, st, fuse, step); break;
     default: return fail(SALVUS_E_INVALID, "bad gather config %d", cfg);
   }
   g_launches++;

@@ -170,72 +170,83 @@ __global__ void batched_source_kernel(int S, int P, const int32_t *__restrict__ 
 }
 
 // Node gather + inverse mass + half-step-velocity update, thread = (NPT
-// consecutive nodes, shot).  CTA = NPB node groups x SC shots.  The NPT
-// nodes' dependent load chains (incidence -> residual) are issued
-// side by side so that more bytes are in flight per thread; the per-node
-// arithmetic and summation order do not depend on NPT.
+// consecutive nodes, four consecutive shots): every field and residual access
+// is 16 bytes per thread, which is what keeps enough bytes in flight behind
+// the dependent chain incidence -> residual.  CTA = NPB node groups x SC
+// shots, SC / 4 * NPB threads.  The NPT nodes' chains are issued side by
+// side.  One shot per thread moved 3.7 of 6.5 TB/s on the edge nodes of 200^2
+// order-4 quads x 256 shots; four took the step from 1075 to 875 us (B200).
+// The per-node arithmetic and summation order do not depend on the split.
 // nodes != nullptr: thread slot t handles node nodes[t] (the edge nodes of
 // the fused form), G is then the list's length.
 template <int SC, int NPB, int NPT>
-__global__ void __launch_bounds__(SC *NPB)
+__global__ void __launch_bounds__(SC / 4 * NPB)
 batched_gather_update_kernel(int64_t G, int S, Incidence inc, const float *__restrict__ r,
                              const float *__restrict__ mi, float *__restrict__ u,
                              float *__restrict__ w, float dt,
                              const int32_t *__restrict__ nodes, int64_t *__restrict__ step) {
   if (step && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *step += 1;
-  const int ny = threadIdx.x / SC, lane = threadIdx.x - ny * SC;
+  constexpr int LN = SC / 4;
+  const int ny = threadIdx.x / LN, lane = threadIdx.x - ny * LN;
   const int64_t g0 = ((int64_t)blockIdx.x * NPB + ny) * NPT;
-  const int s = blockIdx.y * SC + lane;
+  const int s = blockIdx.y * SC + 4 * lane;
   if (g0 >= G || s >= S) return;
-  constexpr int kFast = 4;  // quadrilateral valence bound
-  float uo[NPT], wo[NPT], m[NPT];
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add = [](float4 &x, const float4 &y) { x.x += y.x, x.y += y.y, x.z += y.z, x.w += y.w; };
+  float4 uo[NPT], wo[NPT];
+  float m[NPT];
   int2 h[NPT];
-  int32_t cnt[NPT];
   int64_t gk[NPT];
 #pragma unroll
   for (int k = 0; k < NPT; ++k) {
     const bool live = g0 + k < G;
     const int64_t g = !live ? 0 : nodes ? (int64_t)__ldg(nodes + g0 + k) : g0 + k;
     gk[k] = g;
-    const int64_t i = g * S + s;
-    uo[k] = live ? u[i] : 0.f;
-    wo[k] = live ? w[i] : 0.f;
+    h[k] = live ? __ldg(inc.head + g) : int2{0, -1};
+    uo[k] = live ? *reinterpret_cast<const float4 *>(u + g * S + s) : zero;
+    wo[k] = live ? *reinterpret_cast<const float4 *>(w + g * S + s) : zero;
     m[k] = live ? __ldg(mi + g) : 0.f;
-    h[k] = live ? __ldg(inc.head + g) : int2{0, 0};
-    cnt[k] = !live ? 0 : h[k].y >= -1 ? 1 + (h[k].y >= 0) : -h[k].y;
   }
-  // all incidence indices first, then all residual loads in flight at once
-  int32_t ep[NPT][kFast];
+  auto load = [&](int32_t ep) {
+    return __ldg(reinterpret_cast<const float4 *>(r + (int64_t)ep * S + s));
+  };
+  // summed in ascending element order
+  float4 acc[NPT], second[NPT];
 #pragma unroll
-  for (int k = 0; k < NPT; ++k)
-#pragma unroll
-    for (int q = 0; q < kFast; ++q)
-      ep[k][q] = q >= cnt[k] ? 0 : cnt[k] > 2 ? __ldg(inc.rest + h[k].x + q) : q == 0 ? h[k].x : h[k].y;
-  float rv[NPT][kFast];
-#pragma unroll
-  for (int k = 0; k < NPT; ++k)
-#pragma unroll
-    for (int q = 0; q < kFast; ++q)
-      rv[k][q] = q < cnt[k] ? __ldg(r + (int64_t)ep[k][q] * S + s) : 0.f;
+  for (int k = 0; k < NPT; ++k) {
+    const bool live = g0 + k < G;
+    acc[k] = live && h[k].y >= -1 ? load(h[k].x) : zero;
+    second[k] = live && h[k].y >= 0 ? load(h[k].y) : zero;
+  }
 #pragma unroll
   for (int k = 0; k < NPT; ++k) {
     if (g0 + k >= G) break;
-    const int64_t g = gk[k];
-    // summed in ascending element order
-    float acc = 0.f;
-    if (cnt[k] <= kFast) {
+    float4 sum = zero;
+    add(sum, acc[k]);
+    if (h[k].y >= 0) {
+      add(sum, second[k]);
+    } else if (h[k].y < -1) {
+      constexpr int kBatch = 4;  // the usual valence of a quadrilateral vertex
+      const int32_t q1 = h[k].x - h[k].y;
+      for (int32_t qb = h[k].x; qb < q1; qb += kBatch) {
+        int32_t ep[kBatch];
+        float4 rv[kBatch];
 #pragma unroll
-      for (int q = 0; q < kFast; ++q)
-        if (q < cnt[k]) acc += rv[k][q];
-    } else {
-      for (int32_t q = h[k].x; q < h[k].x + cnt[k]; ++q)
-        acc += __ldg(r + (int64_t)__ldg(inc.rest + q) * S + s);
+        for (int z = 0; z < kBatch; ++z) ep[z] = qb + z < q1 ? __ldg(inc.rest + qb + z) : 0;
+#pragma unroll
+        for (int z = 0; z < kBatch; ++z) rv[z] = qb + z < q1 ? load(ep[z]) : zero;
+#pragma unroll
+        for (int z = 0; z < kBatch; ++z)
+          if (qb + z < q1) add(sum, rv[z]);
+      }
     }
-    float wn = wo[k], un = uo[k];
-    half_step_update(acc, m[k], dt, wn, un);
-    const int64_t i = g * S + s;
-    w[i] = wn;
-    u[i] = un;
+    half_step_update(sum.x, m[k], dt, wo[k].x, uo[k].x);
+    half_step_update(sum.y, m[k], dt, wo[k].y, uo[k].y);
+    half_step_update(sum.z, m[k], dt, wo[k].z, uo[k].z);
+    half_step_update(sum.w, m[k], dt, wo[k].w, uo[k].w);
+    const int64_t i = gk[k] * S + s;
+    *reinterpret_cast<float4 *>(w + i) = wo[k];
+    *reinterpret_cast<float4 *>(u + i) = uo[k];
   }
 }
 
