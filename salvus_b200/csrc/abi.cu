@@ -239,6 +239,14 @@ static int acoustic2(const salvus_mesh *m, const real *rec, const real *u, real 
     using S = QuadColShape<N, EPB>;
     const DMatrix<real> D = dmatrix<real>(m->basis);
     const int32_t *cn = m->d_conn.as<int32_t>();
+    if constexpr (std::is_same<real, float>::value) {
+      if (m->qfactors) {
+        acoustic_quad_affine_kernel<N, EPB><<<blocks_for(m->E, EPB), S::THREADS, 0, s>>>(
+            m->E, m->d_qs32.as<float>(), m->d_qm32.as<float4>(), cn, u, r, D);
+        g_launches++;
+        return check_launch("acoustic quad stiffness");
+      }
+    }
     if (m->physics == SALVUS_ACOUSTIC) {
       acoustic_quad_col_kernel<N, EPB, real><<<blocks_for(m->E, EPB), S::THREADS, 0, s>>>(
           m->E, rec, cn, u, r, D);
@@ -568,7 +576,7 @@ static int build_records(salvus_mesh *m, DeviceBuffer &out, DeviceBuffer &mass_l
   geometry_kernel<real, kPack><<<blocks_for(total, 128), 128, 0, m->stream>>>(
       m->E, m->dim, m->n, m->P, m->physics, rw, m->d_vtx.as<double>(), m->d_par.as<double>(),
       m->d_conn.as<int32_t>(), gll, out.as<real>(), mass_local.as<double>(),
-      m->d_cls_k.as<int32_t>(), m->n_fluid, m->ti);
+      m->d_cls_k.as<int32_t>(), m->n_fluid, m->ti, m->qaffine);
   g_launches++;
   return check_launch("geometry");
 }
@@ -714,6 +722,20 @@ static int mesh_setup_device(salvus_mesh *m) {
     if ((rc = check_launch("affine records"))) return rc;
   } else if ((rc = build_records<float, true>(m, m->d_rec32, mass_local))) {
     return rc;
+  }
+  if (m->qfactors) {
+    if ((rc = m->d_qs32.alloc(sizeof(float) * EP)) || (rc = m->d_qm32.alloc(sizeof(float4) * m->E)))
+      return rc;
+    GllTable gll{};
+    for (int i = 0; i < m->n; ++i) {
+      gll.xi[i] = m->basis.xi[i];
+      gll.w[i] = m->basis.w[i];
+    }
+    quad_affine_factors_kernel<<<blocks_for(EP, 128), 128, 0, m->stream>>>(
+        m->E, m->n, m->P, m->d_vtx.as<double>(), m->d_par.as<double>(), gll, m->d_qs32.as<float>(),
+        m->d_qm32.as<float4>());
+    g_launches++;
+    if ((rc = check_launch("quad factors"))) return rc;
   }
   // the node list of the fused steps (interior_free_nodes, at creation)
   if (m->n_gnodes > 0) {
@@ -1730,8 +1752,8 @@ static int group_fill(salvus_group *g) {
     int rc = ready(p);
     if (rc) return rc;
     GroupSlot &s = g->slots[k];
-    s.rec = m->d_rec32.as<float>();
-    s.jac = m->affine ? m->d_jac32.as<float>() : nullptr;
+    s.rec = m->qfactors ? m->d_qs32.as<float>() : m->d_rec32.as<float>();
+    s.jac = m->affine ? m->d_jac32.as<float>() : m->qfactors ? m->d_qm32.as<float>() : nullptr;
     s.conn = m->d_conn.as<int32_t>();
     s.inc_off = m->d_inc_off.as<int32_t>();
     s.inc_idx = m->d_inc_idx.as<int32_t>();
@@ -2156,6 +2178,21 @@ int salvus_mesh_create(const salvus_mesh_desc *d, int device, salvus_mesh **out)
     }
     m->affine = affine;
     m->affine64 = affine && affine64;
+  }
+  if (m->shape == SALVUS_QUAD && m->physics != SALVUS_ELASTIC2D) {
+    // every element a parallelogram: opposite edges equal to 1e-9 of the
+    // shorter edge, which bounds how far the Jacobian varies over the element
+    // (FP32 rounds it at 6e-8)
+    bool para = true;
+    for (int64_t e = 0; e < m->E && para; ++e) {
+      const double *v = m->vtx.data() + e * 8;
+      const double off = std::hypot((v[0] - v[2]) + (v[4] - v[6]), (v[1] - v[3]) + (v[5] - v[7]));
+      const double a = std::hypot(v[2] - v[0], v[3] - v[1]), b = std::hypot(v[6] - v[0], v[7] - v[1]);
+      para = off <= 1e-9 * std::min(a, b);
+    }
+    m->qaffine = para;
+    m->qfactors = para && m->physics == SALVUS_ACOUSTIC &&
+                  !(d->reserved & SALVUS_MESH_PER_POINT_GEOMETRY);
   }
   if ((rc = flatten_mesh(m.get(), d->cells, d->n_vertices))) return rc;
   if (m->physics == SALVUS_COUPLED2D && (rc = setup_coupled(m.get(), d->cells))) return rc;

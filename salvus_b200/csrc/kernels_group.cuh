@@ -26,8 +26,9 @@
 namespace salvus {
 
 struct GroupSlot {
-  // mesh (hexahedra: jac != nullptr for parallelepiped meshes, whose rec holds
-  // the material planes of kernels_hex_affine.cuh)
+  // mesh (jac != nullptr for meshes of parallelepipeds, whose rec holds the
+  // material planes of kernels_hex_affine.cuh, and of parallelograms, whose rec
+  // and jac are the factors of acoustic_quad_affine_kernel)
   const float *rec, *jac;
   const int32_t *conn, *inc_off, *inc_idx;
   Incidence inc;  // quadrilaterals
@@ -64,6 +65,17 @@ __device__ __forceinline__ void group_hex_body(const GroupSlot &m, int64_t bid,
   }
 }
 
+template <int N>
+__device__ __forceinline__ void group_quad_body(const GroupSlot &m, int64_t bid,
+                                                const DMatrix<float> &Dm) {
+  constexpr int EPB = quad_col_epb<N>();
+  if (m.jac)
+    acoustic_quad_col_body<N, EPB, float, 1, false, true>(
+        bid, m.E, m.rec, m.conn, m.u, m.r, Dm, nullptr, reinterpret_cast<const float4 *>(m.jac));
+  else
+    acoustic_quad_col_body<N, EPB, float>(bid, m.E, m.rec, m.conn, m.u, m.r, Dm);
+}
+
 // owner[b]: the member whose CTA range of this launch holds CTA b (a table
 // per stage, filled on the host; one load instead of a search).
 
@@ -72,8 +84,7 @@ __global__ void __launch_bounds__(QuadColShape<N, quad_col_epb<N>()>::THREADS)
 group_quad_acoustic_stiffness(const GroupSlot *__restrict__ slots,
                               const int32_t *__restrict__ owner, DMatrix<float> Dm) {
   const GroupSlot &m = slots[owner[blockIdx.x]];
-  acoustic_quad_col_body<N, quad_col_epb<N>(), float>(blockIdx.x - m.b_stiff, m.E, m.rec, m.conn,
-                                                       m.u, m.r, Dm);
+  group_quad_body<N>(m, blockIdx.x - m.b_stiff, Dm);
 }
 
 template <int N, int EPB>
@@ -203,7 +214,7 @@ group_persistent_step(const GroupSlot *__restrict__ slots, const GroupCounts *__
           if constexpr (kHex)
             group_hex_body<N, EPB>(m, b, Dm);
           else
-            acoustic_quad_col_body<N, quad_col_epb<N>(), float>(b, m.E, m.rec, m.conn, m.u, m.r, Dm);
+            group_quad_body<N>(m, b, Dm);
           __syncthreads();
         }
         break;
@@ -303,7 +314,7 @@ group_partitioned_step(const GroupSlot *__restrict__ slots, const GroupPart *__r
     if constexpr (kHex)
       group_hex_body<N, EPB>(m, k, Dm);
     else
-      acoustic_quad_col_body<N, quad_col_epb<N>(), float>(k, m.E, m.rec, m.conn, m.u, m.r, Dm);
+      group_quad_body<N>(m, k, Dm);
     __syncthreads();
   }
   arrive(&gb->stiff_done);
