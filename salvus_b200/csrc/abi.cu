@@ -824,6 +824,7 @@ static int upload_sources(salvus_problem *p) {
     std::vector<double> par(3 * ns), w(ns * m->P * p->c);
     std::vector<int32_t> shot_off(p->shots_pad + 1, 0), tile;
     std::vector<int4> node;
+    std::vector<uint8_t> has(p->shots > 1 ? (size_t)m->E : 0, 0);
     for (size_t k = 0; k < ns; ++k) {
       const auto &src = p->srcs[order[k]];
       el[k] = src.elem;
@@ -834,6 +835,7 @@ static int upload_sources(salvus_problem *p) {
       shot_off[src.desc.shot + 1]++;
       // distinct source elements (fused hexahedron step)
       if (p->shots == 1 && (ue.empty() || ue.back() != src.elem)) ue.push_back(src.elem);
+      if (p->shots > 1) has[(size_t)src.elem] = 1;
     }
     for (int s = 0; s < p->shots_pad; ++s) shot_off[s + 1] += shot_off[s];
     if (p->shots == 1) source_tiles(m, el, tile, node);
@@ -852,6 +854,7 @@ static int upload_sources(salvus_problem *p) {
     const size_t o_so = put(shot_off.data(), sizeof(int32_t) * shot_off.size());
     const size_t o_t = put(tile.data(), sizeof(int32_t) * tile.size());
     const size_t o_n = put(node.data(), sizeof(int4) * node.size());
+    const size_t o_h = put(has.data(), has.size());
     const size_t o_stf = put(nullptr, sizeof(double) * ns);
     int rc = p->d_src.alloc(img.size());
     if (rc) return rc;
@@ -863,6 +866,7 @@ static int upload_sources(salvus_problem *p) {
     p->shot_off = (const int32_t *)(d + o_so);
     p->src_tile = (const int32_t *)(d + o_t);
     p->src_node = (const int4 *)(d + o_n);
+    p->has_src = (const uint8_t *)(d + o_h);
     p->stf = (double *)(d + o_stf);
     p->n_src_uelem = (int)ue.size();
     SALVUS_CUDA(cudaMemcpyAsync(d, img.data(), img.size(), cudaMemcpyHostToDevice, p->stream));
@@ -1122,10 +1126,23 @@ static int step_fused_t(salvus_problem *p, bool store_a) {
 // ---------------------------------------------------------------------------
 // shot-batched step (FP32 acoustic quads)
 struct BatchCfg {
-  int sc, epc, npt;  // shot lanes, elements / node groups per CTA, nodes per thread
+  int sc, epc, npt;  // shots, elements / node groups per CTA, nodes per thread
 };
+// Stiffness: the third number is the shots per thread; {0, 1, 2} takes CTAs of
+// pair_shots.  Below 64 shots its CTAs would be less than a warp.
 static const BatchCfg kStiffCfg[] = {{32, 1, 1}, {32, 2, 1}, {32, 4, 1}, {64, 1, 1},
-                                     {64, 2, 1}, {128, 1, 1}, {128, 2, 1}, {256, 1, 1}};
+                                     {128, 1, 1}, {0, 1, 2}};
+// shots per CTA of {0, 1, 2}: the most 32-shot groups, up to eight, that
+// divide the padded shots
+static int pair_shots(int shots_pad) {
+  for (int k = 8; k > 1; --k)
+    if (shots_pad % (32 * k) == 0) return 32 * k;
+  return 32;
+}
+static bool stiff_cfg_fits(int cfg, int shots_pad) {
+  const int sc = kStiffCfg[cfg].sc;
+  return sc ? shots_pad % sc == 0 : pair_shots(shots_pad) >= 64;
+}
 static const BatchCfg kGatherCfg[] = {{32, 16, 1}, {32, 32, 1}, {64, 8, 1}, {64, 16, 1},
                                       {128, 4, 1}, {128, 8, 1}, {256, 2, 1}, {256, 4, 1},
                                       {32, 16, 2}, {64, 8, 2},  {128, 4, 2}, {256, 2, 2}};
@@ -1142,22 +1159,24 @@ static bool batch_fusion(const salvus_problem *p) {
   return !(s && std::strcmp(s, "unfused") == 0);
 }
 
-template <int N, int SC, int EPC>
+template <int N, int SC, int EPC, int V>
 static void launch_qb(const salvus_problem *p, cudaStream_t st, bool fuse) {
   const salvus_mesh *m = p->mesh;
-  dim3 grid((unsigned)((m->E + EPC - 1) / EPC), (unsigned)(p->shots_pad / SC));
+  const int sc = SC ? SC : pair_shots(p->shots_pad);
+  dim3 grid((unsigned)((m->E + EPC - 1) / EPC), (unsigned)(p->shots_pad / sc));
   BatchInterior bi{};
   if (fuse) {
     bi.mi = m->d_mi32.as<float>();
     bi.w = F<float>(p->d_v);
     bi.dt = (float)p->dt;
-    bi.shot_off = p->srcs.empty() ? nullptr : p->shot_off;
+    bi.shot_off = p->shot_off;
     bi.src_elem = p->src_elem;
-    quad_acoustic_batched_kernel<N, SC, EPC, true><<<grid, SC * EPC, 0, st>>>(
+    bi.has_src = p->srcs.empty() ? nullptr : p->has_src;
+    quad_acoustic_batched_kernel<N, SC, EPC, V, true><<<grid, sc / V * EPC, 0, st>>>(
         m->E, p->shots_pad, m->d_rec32.as<float>(), F<float>(p->d_u), F<float>(p->d_r),
         dmatrix<float>(m->basis), bi);
   } else {
-    quad_acoustic_batched_kernel<N, SC, EPC, false><<<grid, SC * EPC, 0, st>>>(
+    quad_acoustic_batched_kernel<N, SC, EPC, V, false><<<grid, sc / V * EPC, 0, st>>>(
         m->E, p->shots_pad, m->d_rec32.as<float>(), F<float>(p->d_u), F<float>(p->d_r),
         dmatrix<float>(m->basis), bi);
   }
@@ -1166,14 +1185,12 @@ static void launch_qb(const salvus_problem *p, cudaStream_t st, bool fuse) {
 template <int N>
 static int launch_qb_cfg(const salvus_problem *p, int cfg, cudaStream_t st, bool fuse) {
   switch (cfg) {
-    case 0: launch_qb<N, 32, 1>(p, st, fuse); break;
-    case 1: launch_qb<N, 32, 2>(p, st, fuse); break;
-    case 2: launch_qb<N, 32, 4>(p, st, fuse); break;
-    case 3: launch_qb<N, 64, 1>(p, st, fuse); break;
-    case 4: launch_qb<N, 64, 2>(p, st, fuse); break;
-    case 5: launch_qb<N, 128, 1>(p, st, fuse); break;
-    case 6: launch_qb<N, 128, 2>(p, st, fuse); break;
-    case 7: launch_qb<N, 256, 1>(p, st, fuse); break;
+    case 0: launch_qb<N, 32, 1, 1>(p, st, fuse); break;
+    case 1: launch_qb<N, 32, 2, 1>(p, st, fuse); break;
+    case 2: launch_qb<N, 32, 4, 1>(p, st, fuse); break;
+    case 3: launch_qb<N, 64, 1, 1>(p, st, fuse); break;
+    case 4: launch_qb<N, 128, 1, 1>(p, st, fuse); break;
+    case 5: launch_qb<N, 0, 1, 2>(p, st, fuse); break;
     default: return fail(SALVUS_E_INVALID, "bad batch config %d", cfg);
   }
   g_launches++;
@@ -1253,7 +1270,7 @@ static int autotune(salvus_problem *p) {
   if (env) {
     int a = -1, b = -1;
     if (std::sscanf(env, "%d,%d", &a, &b) == 2 && a >= 0 && a < kNumStiffCfg && b >= 0 &&
-        b < kNumGatherCfg && p->shots_pad % kStiffCfg[a].sc == 0 && p->shots_pad % kGatherCfg[b].sc == 0) {
+        b < kNumGatherCfg && stiff_cfg_fits(a, p->shots_pad) && p->shots_pad % kGatherCfg[b].sc == 0) {
       p->tune_stiff = a;
       p->tune_gather = b;
       return SALVUS_OK;
@@ -1290,7 +1307,7 @@ static int autotune(salvus_problem *p) {
     cudaMemsetAsync(p->d_u.ptr, 0, nf, p->stream);
     cudaMemsetAsync(p->d_v.ptr, 0, nf, p->stream);
     for (int c = 0; c < kNumStiffCfg && rc == SALVUS_OK; ++c) {
-      if (p->shots_pad % kStiffCfg[c].sc) continue;
+      if (!stiff_cfg_fits(c, p->shots_pad)) continue;
       float t = time_it([&] { return batched_stiffness(p, c, p->stream, fuse); });
       if (t < bs) { bs = t; cs = c; }
     }
@@ -3062,7 +3079,9 @@ int salvus_problem_autotune(salvus_problem *p, int32_t *stiff_shot_lanes, int32_
     if (gather_nodes) *gather_nodes = 256;
     return SALVUS_OK;
   }
-  if (stiff_shot_lanes) *stiff_shot_lanes = kStiffCfg[p->tune_stiff].sc;
+  if (stiff_shot_lanes)
+    *stiff_shot_lanes = kStiffCfg[p->tune_stiff].sc ? kStiffCfg[p->tune_stiff].sc
+                                                    : pair_shots(p->shots_pad);
   if (stiff_elements) *stiff_elements = kStiffCfg[p->tune_stiff].epc;
   if (gather_shot_lanes) *gather_shot_lanes = kGatherCfg[p->tune_gather].sc;
   if (gather_nodes) *gather_nodes = kGatherCfg[p->tune_gather].epc * kGatherCfg[p->tune_gather].npt;

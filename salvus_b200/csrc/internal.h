@@ -209,6 +209,7 @@ struct salvus_problem {
   const double *src_par = nullptr, *src_wts = nullptr;
   const int32_t *shot_off = nullptr, *src_tile = nullptr;
   const int4 *src_node = nullptr;
+  const uint8_t *has_src = nullptr;  // batched: elements with a source of any shot
   double *stf = nullptr;
   int n_src_uelem = 0;
   bool stf_ready = false;

@@ -32,6 +32,7 @@ struct BatchInterior {
   float dt;
   const int32_t *shot_off;  // sources of shot s: [shot_off[s], shot_off[s + 1])
   const int64_t *src_elem;
+  const uint8_t *has_src;  // per element: any shot has a source in it (null: no sources)
 };
 
 // half-step-velocity update of one node (one shot): w += dt a; u += dt w,
@@ -42,15 +43,35 @@ __device__ __forceinline__ void half_step_update(float acc, float m, float dt, f
   u = __fmaf_rn(dt, w, u);
 }
 
-// One thread = one shot of one quad element; the element's n^2 values of
-// that shot live in registers, so the tensor-product contractions need no
-// shared memory.  CTA = EPC elements x SC shots.
-template <int N, int SC, int EPC, bool kFuse = false>
-__global__ void __launch_bounds__(SC *EPC)
+// One thread = V consecutive shots of one quad element; the element's n^2
+// values of those shots live in registers, so the tensor-product contractions
+// need no shared memory.  CTA = EPC elements x SC shots, SC / V * EPC threads
+// (SC = 0: one element, V shots for each thread of the launch).
+// The element is walked row by row: a row's fluxes are formed, spread over the
+// outputs of their columns and dropped, so that values and outputs (2 n^2 a
+// shot) are all that lives throughout; with both flux fields kept the kernel
+// could not take two shots.  Two shots per thread make every access 8 bytes
+// and halve the address and record work; the register caps below keep enough
+// warps per SM.  200^2 order 4 x 256 shots, fused launch: 564 us with one shot
+// per thread and both flux fields, 446 with two (512 threads per SM; without
+// the cap 533, 163 registers); 130^2 order 3, a step: 234 -> 217 us (768
+// threads per SM; 512: 231).
+template <int N, int SC, int EPC, int V>
+constexpr int batched_ctas_per_sm() {
+  constexpr int threads = SC ? SC / V * EPC : 128;
+  constexpr int pair = N <= 2 ? 1024 : N == 3 ? 768 : N == 4 ? 512 : 256;
+  constexpr int one = N <= 2 ? 1536 : N == 3 ? 1024 : N == 4 ? 896 : N == 5 ? 512 : 384;
+  constexpr int resident = V == 2 ? pair : one;  // threads per SM
+  constexpr int ctas = resident / threads > 0 ? resident / threads : 1;
+  return ctas < 32 ? ctas : 32;
+}
+template <int N, int SC, int EPC, int V, bool kFuse = false>
+__global__ void __launch_bounds__(SC ? SC / V * EPC : 128, batched_ctas_per_sm<N, SC, EPC, V>())
 quad_acoustic_batched_kernel(int64_t E, int S, const float *__restrict__ rec,
                              float *__restrict__ u, float *__restrict__ r,
                              DMatrix<float> Dm, BatchInterior bi) {
   constexpr int n = N + 1, P = n * n;
+  const int LN = SC ? SC / V : (int)blockDim.x;
   __shared__ float4 sg[EPC * P];  // G00 G01 G11 conn of the CTA's elements
   const int64_t e0 = (int64_t)blockIdx.x * EPC;
   for (int q = threadIdx.x; q < EPC * P; q += blockDim.x) {
@@ -59,71 +80,96 @@ quad_acoustic_batched_kernel(int64_t E, int S, const float *__restrict__ rec,
                    : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
-  const int ey = threadIdx.x / SC, lane = threadIdx.x - ey * SC;
+  const int ey = threadIdx.x / LN, lane = threadIdx.x - ey * LN;
   const int64_t e = e0 + ey;
-  const int s = blockIdx.y * SC + lane;
+  const int s = (blockIdx.y * LN + lane) * V;
   if (e >= E || s >= S) return;
   const float4 *g = sg + ey * P;
-  float uu[P];
-#pragma unroll
-  for (int p = 0; p < P; ++p) {
-    // the fused form writes u of interior nodes during the launch: coherent loads
-    const float *up = u + (int64_t)__float_as_int(g[p].w) * S + s;
-    uu[p] = kFuse ? *up : __ldg(up);
-  }
-  // fused form: whether one of this shot's sources sits in this element (then
-  // the unfused form for its interior points), and the interior nodes' w,
-  // loaded before the arithmetic so that their latency overlaps it (w is
-  // written below; the read-only inverse mass is read where it is used)
-  bool fuse_here = kFuse;
-  float wpre[P];
-  if constexpr (kFuse) {
-    if (bi.shot_off)
-      for (int k = bi.shot_off[s]; k < bi.shot_off[s + 1] && fuse_here; ++k)
-        fuse_here = __ldg(bi.src_elem + k) != e;
-    if (fuse_here) {
-#pragma unroll
-      for (int p = 0; p < P; ++p) {
-        const int i = p % n, j = p / n;
-        if (i < 1 || i > n - 2 || j < 1 || j > n - 2) continue;
-        wpre[p] = bi.w[(int64_t)__float_as_int(g[p].w) * S + s];
-      }
-    }
-  }
-  float Fr[P], Fs[P];
-#pragma unroll
-  for (int p = 0; p < P; ++p) {
+  struct alignas(4 * V) Shots {
+    float v[V];
+  };
+  auto at = [&](float *field, int p) -> Shots & {
+    return *reinterpret_cast<Shots *>(field + (int64_t)__float_as_int(g[p].w) * S + s);
+  };
+  auto interior = [](int p) {
     const int i = p % n, j = p / n;
-    float gr = 0.f, gs = 0.f;
+    return i >= 1 && i <= n - 2 && j >= 1 && j <= n - 2;
+  };
+  // plain (coherent) loads: the fused form writes u of interior nodes
+  Shots uu[P];
 #pragma unroll
-    for (int l = 0; l < n; ++l) {
-      gr += Dm.d[i * n + l] * uu[l + n * j];
-      gs += Dm.d[j * n + l] * uu[i + n * l];
+  for (int p = 0; p < P; ++p) uu[p] = at(u, p);
+  // fused form: the interior nodes' w, and whether one of a shot's sources
+  // sits in this element (then the unfused form for its interior points).
+  // Nearly no element holds a source of any shot, and one byte says so; with
+  // the shots' source lists searched by every thread the order-4 launch on
+  // 200^2 x 256 shots took 535 us
+  Shots wpre[P];
+  bool fuse[V], all = kFuse;
+  if constexpr (kFuse) {
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+      if (interior(p)) wpre[p] = at(bi.w, p);
+    const bool search = bi.has_src && __ldg(bi.has_src + e);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      fuse[v] = true;
+      if (search)
+        for (int k = bi.shot_off[s + v]; k < bi.shot_off[s + v + 1] && fuse[v]; ++k)
+          fuse[v] = __ldg(bi.src_elem + k) != e;
+      all = all && fuse[v];
     }
-    const float4 G = g[p];
-    Fr[p] = G.x * gr + G.y * gs;
-    Fs[p] = G.y * gr + G.z * gs;
   }
+  float o[V][P];
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+#pragma unroll
+    for (int p = 0; p < P; ++p) o[v][p] = 0.f;
+#pragma unroll
+  for (int j = 0; j < n; ++j)
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      float Fr[n];
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        float gr = 0.f, gs = 0.f;
+#pragma unroll
+        for (int l = 0; l < n; ++l) {
+          gr += Dm.d[i * n + l] * uu[l + n * j].v[v];
+          gs += Dm.d[j * n + l] * uu[i + n * l].v[v];
+        }
+        const float4 G = g[i + n * j];
+        Fr[i] = G.x * gr + G.y * gs;
+        const float Fs = G.y * gr + G.z * gs;
+#pragma unroll
+        for (int m = 0; m < n; ++m) o[v][i + n * m] += Dm.d[j * n + m] * Fs;
+      }
+#pragma unroll
+      for (int i = 0; i < n; ++i)
+#pragma unroll
+        for (int l = 0; l < n; ++l) o[v][i + n * j] += Dm.d[l * n + i] * Fr[l];
+    }
   float *out = r + (e * P) * S + s;
 #pragma unroll
   for (int p = 0; p < P; ++p) {
-    const int i = p % n, j = p / n;
-    float o = 0.f;
+    if (!interior(p) || !all) {
+      Shots x;
 #pragma unroll
-    for (int l = 0; l < n; ++l) {
-      o += Dm.d[l * n + i] * Fr[l + n * j];
-      o += Dm.d[l * n + j] * Fs[i + n * l];
-    }
-    if (!fuse_here || i < 1 || i > n - 2 || j < 1 || j > n - 2) {
-      out[(int64_t)p * S] = -o;
-      continue;
+      for (int v = 0; v < V; ++v) x.v[v] = -o[v][p];
+      *reinterpret_cast<Shots *>(out + (int64_t)p * S) = x;
     }
     if constexpr (kFuse) {
-      const int64_t x = (int64_t)__float_as_int(g[p].w) * S + s;
-      float wv = wpre[p], uv = uu[p];
-      half_step_update(__fadd_rn(0.f, -o), __ldg(bi.mi + __float_as_int(g[p].w)), bi.dt, wv, uv);
-      bi.w[x] = wv;
-      u[x] = uv;
+      if (interior(p)) {
+        // a shot left to the source kernel keeps its u and w
+        Shots wv = wpre[p], uv = uu[p];
+        const float m = __ldg(bi.mi + __float_as_int(g[p].w));
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+          if (fuse[v])
+            half_step_update(__fadd_rn(0.f, -o[v][p]), m, bi.dt, wv.v[v], uv.v[v]);
+        at(bi.w, p) = wv;
+        at(u, p) = uv;
+      }
     }
   }
 }
