@@ -2287,60 +2287,43 @@ int salvus_mesh_max_eigenvalue(salvus_mesh *m, int32_t iters, uint64_t seed, dou
   if (m->fp32_only) return fail(SALVUS_E_STATE, "the eigenvalue estimate needs the FP64 records");
   SALVUS_CUDA(cudaSetDevice(m->device));
   const int64_t N = m->G * m->c;
-  DeviceBuffer x, y, r, mass, part;
+  // partial sums of the three dot products, then the estimate
+  DeviceBuffer x, y, r, part;
   int rc;
   if ((rc = x.alloc(8 * N)) || (rc = y.alloc(8 * N)) || (rc = r.alloc(8 * m->E * m->P * m->c)) ||
-      (rc = mass.alloc(8 * m->G)) || (rc = part.alloc(8 * 1024)))
+      (rc = part.alloc(sizeof(double) * (3 * kEigBlocks + 1))))
     return rc;
-  std::vector<double> h(N), mh(m->G);
+  std::vector<double> h(N);
   std::mt19937_64 rng(seed ? seed : 1);
   std::uniform_real_distribution<double> U(-0.5, 0.5);
   for (auto &v : h) v = U(rng);
-  for (int64_t g = 0; g < m->G; ++g) mh[g] = 1.0 / m->mi[g];
   SALVUS_CUDA(cudaMemcpyAsync(x.ptr, h.data(), 8 * N, cudaMemcpyHostToDevice, m->stream));
-  SALVUS_CUDA(cudaMemcpyAsync(mass.ptr, mh.data(), 8 * m->G, cudaMemcpyHostToDevice, m->stream));
-  const int nb = 512;
-  std::vector<double> hp(nb);
-  auto dot = [&](const double *a, const double *b, double &out) -> int {
-    dot_kernel<double><<<nb, 256, 0, m->stream>>>(N, m->c, a, b, mass.as<double>(), part.as<double>());
-    g_launches++;
-    SALVUS_CUDA(cudaMemcpyAsync(hp.data(), part.ptr, 8 * nb, cudaMemcpyDeviceToHost, m->stream));
-    SALVUS_CUDA(cudaStreamSynchronize(m->stream));
-    double s = 0;
-    for (int i = 0; i < nb; ++i) s += hp[i];
-    out = s;
-    return SALVUS_OK;
-  };
-  double lam = 0;
+  double *lam = part.as<double>() + 3 * kEigBlocks;
+  SALVUS_CUDA(cudaMemsetAsync(lam, 0, sizeof(double), m->stream));
+  // Nothing of an iteration comes back to the host: four launches, where three
+  // dot products each copied and summed 512 partials there
   for (int it = 0; it < iters; ++it) {
     if ((rc = launch_stiffness<double>(m, m->d_rec64.as<double>(), x.as<double>(), r.as<double>(),
                                        m->stream)))
       return rc;
-    // y = -gather(r) = K x ; then M^-1
-    by_components(m->c, [&](auto cc) {
+    rc = by_components(m->c, [&](auto cc) {
       constexpr int C = decltype(cc)::value;
       gather_kernel<double, C, 1><<<blocks_for(m->G, 256), 256, 0, m->stream>>>(
           m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), r.as<double>(), nullptr,
           nullptr, nullptr, nullptr, y.as<double>(), 0.0);
-      inverse_mass_kernel<double, C><<<blocks_for(N, 256), 256, 0, m->stream>>>(
-          m->G, m->d_mi64.as<double>(), y.as<double>());
+      eig_dots_kernel<C><<<kEigBlocks, kEigThreads, 0, m->stream>>>(
+          N, m->d_mi64.as<double>(), x.as<double>(), y.as<double>(), part.as<double>());
       return SALVUS_OK;
     });
-    g_launches += 2;
-    scale_kernel<double><<<blocks_for(N, 256), 256, 0, m->stream>>>(N, y.as<double>(), -1.0);
-    g_launches++;
-    double xy, xx, yy;
-    if ((rc = dot(x.as<double>(), y.as<double>(), xy)) || (rc = dot(x.as<double>(), x.as<double>(), xx)) ||
-        (rc = dot(y.as<double>(), y.as<double>(), yy)))
-      return rc;
-    lam = xy / xx;
+    if (rc) return rc;
+    eig_scale_kernel<<<kEigBlocks, kEigThreads, 0, m->stream>>>(N, part.as<double>(),
+                                                                y.as<double>(), lam);
+    g_launches += 3;
+    if ((rc = check_launch("eigenvalue iteration"))) return rc;
     std::swap(x.ptr, y.ptr);
-    scale_kernel<double><<<blocks_for(N, 256), 256, 0, m->stream>>>(N, x.as<double>(),
-                                                                     1.0 / std::sqrt(yy));
-    g_launches++;
   }
+  SALVUS_CUDA(cudaMemcpyAsync(lam_out, lam, sizeof(double), cudaMemcpyDeviceToHost, m->stream));
   SALVUS_CUDA(cudaStreamSynchronize(m->stream));
-  *lam_out = lam;
   return SALVUS_OK;
 }
 
