@@ -325,7 +325,17 @@ static int acoustic2(const salvus_mesh *m, const real *rec, const real *u, real 
 }
 template <int N, typename real>
 static int acoustic3(const salvus_mesh *m, const real *rec, const real *u, real *r, cudaStream_t s) {
-  return launch_acoustic<3, N, real>(m, rec, u, r, s);
+  // order 1: one thread per point (60^3: FP32 16.7 us a step against 16.9, FP64
+  // 30.7 against 41.4)
+  if constexpr (N >= 2) {
+    using T = AcousticHexCol<N, real>;
+    acoustic_hex_col_kernel<N, real><<<blocks_for(m->E, T::EPB), T::Shape::THREADS, 0, s>>>(
+        m->E, rec, m->d_conn.as<int32_t>(), u, r, dmatrix<real>(m->basis));
+    g_launches++;
+    return check_launch("acoustic stiffness");
+  } else {
+    return launch_acoustic<3, N, real>(m, rec, u, r, s);
+  }
 }
 
 // P3 simplices on CUDA cores

@@ -44,15 +44,16 @@ template <> struct HexColPad<5> { static constexpr int A = 5, B = 29, R = 25; };
 template <> struct HexColPad<6> { static constexpr int A = 6, B = 37, R = 4; };
 template <> struct HexColPad<7> { static constexpr int A = 7, B = 52, R = 17; };
 
-template <int N, int EPB_, typename real>
+// NC components per node.
+template <int N, int EPB_, typename real, int NC = 3>
 struct HexColShape {
   static constexpr int n = N + 1, n2 = n * n, P = n2 * n;
   static constexpr int EPB = EPB_;
   static constexpr int THREADS = ((EPB * n2 + 31) / 32) * 32;
   static constexpr int A = HexColPad<n>::A, B = HexColPad<n>::B;
   static constexpr int PL = (n - 1) * (1 + A + B) + 1;  // words of one component
-  static constexpr int ES = 3 * PL + ((HexColPad<n>::R - 3 * PL % 32) + 32) % 32;
-  static constexpr int ARR = EPB * ES;  // words of one array (three components)
+  static constexpr int ES = NC * PL + ((HexColPad<n>::R - NC * PL % 32) + 32) % 32;
+  static constexpr int ARR = EPB * ES;  // words of one array (all components)
   static constexpr size_t SMEM = sizeof(real) * (size_t)3 * ARR;
 };
 
@@ -62,17 +63,17 @@ struct HexColShape {
 // in the same bank: a warp takes one line of each bank, the banks with the
 // most lines left first, and a second one only where the warps after it could
 // not hold what is left.
-template <int N, int EPB>
+template <int N, int EPB, int NC = 3>
 struct HexLines {
-  using S = HexColShape<N, EPB, float>;
+  using S = HexColShape<N, EPB, float, NC>;
   static constexpr uint16_t kNone = 0xffff;
   uint16_t r[S::THREADS], s[S::THREADS];
 };
-template <int N, int EPB>
-constexpr HexLines<N, EPB> make_hex_lines() {
-  using S = HexColShape<N, EPB, float>;
+template <int N, int EPB, int NC = 3>
+constexpr HexLines<N, EPB, NC> make_hex_lines() {
+  using S = HexColShape<N, EPB, float, NC>;
   constexpr int n = S::n, W = S::THREADS / 32, L = EPB * S::n2;
-  HexLines<N, EPB> h{};
+  HexLines<N, EPB, NC> h{};
   for (int dir = 0; dir < 2; ++dir) {
     uint16_t *out = dir == 0 ? h.r : h.s;
     for (int t = 0; t < S::THREADS; ++t) out[t] = HexLines<N, EPB>::kNone;
@@ -103,21 +104,21 @@ constexpr HexLines<N, EPB> make_hex_lines() {
   }
   return h;
 }
-template <int N, int EPB>
-__device__ const HexLines<N, EPB> kHexLines = make_hex_lines<N, EPB>();
+template <int N, int EPB, int NC = 3>
+__device__ const HexLines<N, EPB, NC> kHexLines = make_hex_lines<N, EPB, NC>();
 
-// The three components' lines: out[m] = sum_l D[m][l] in[l] (kT: D[l][m]),
+// The NC components' lines: out[m] = sum_l D[m][l] in[l] (kT: D[l][m]),
 // every load before the first store (they may alias for the compiler, and in
 // the divergence they do).
-template <int n, int stride, int PL, bool kT, typename real>
+template <int n, int stride, int PL, bool kT, int NC = 3, typename real>
 __device__ __forceinline__ void line_apply(const real *in, real *out, const DMatrix<real> &Dm) {
-  real v[3][n];
+  real v[NC][n];
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
+  for (int c = 0; c < NC; ++c)
 #pragma unroll
     for (int l = 0; l < n; ++l) v[c][l] = in[c * PL + l * stride];
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
+  for (int c = 0; c < NC; ++c)
 #pragma unroll
     for (int m = 0; m < n; ++m) {
       real acc = 0;
@@ -340,6 +341,78 @@ elastic_hex_col64_kernel(int64_t E, const double *__restrict__ jac, const double
                          double *__restrict__ r, DMatrix<double> Dm) {
   elastic_hex_col_body<N, HexCol64<N, TI, kAffine>::EPB, double, TI, kAffine, false>(
       blockIdx.x, E, jac, rec, conn, u, r, Dm, HexInteriorUpdate{});
+}
+
+// Acoustic hexahedra of orders 2 and up (Scalar.cpp:58-71) by the same line
+// exchange: G = w detJ vp^2 invJ^T invJ (six products) per point, records as in
+// load_acoustic_rec.  One thread per point read 6 n shared words per point,
+// here 13 and the t direction in registers.  Per step, FP32 / FP64 (B200, us):
+// 24^3 order 4 28.4 -> 20.1 / 53.1 -> 37.4, 15^3 order 6 24.3 -> 15.7 / 42.9 ->
+// 26.8, 40^3 order 2 23.4 -> 18.0 / 42.6 -> 34.7.
+template <int N, typename real>
+struct AcousticHexCol {
+  static constexpr int n2 = (N + 1) * (N + 1);
+  static constexpr int EPB = 128 / n2 > 0 ? 128 / n2 : 1;
+  using Shape = HexColShape<N, EPB, real, 1>;
+};
+template <int N, typename real>
+__global__ void __launch_bounds__(AcousticHexCol<N, real>::Shape::THREADS)
+acoustic_hex_col_kernel(int64_t E, const real *__restrict__ rec, const int32_t *__restrict__ conn,
+                        const real *__restrict__ u, real *__restrict__ r, DMatrix<real> Dm) {
+  constexpr int EPB = AcousticHexCol<N, real>::EPB;
+  using S = typename AcousticHexCol<N, real>::Shape;
+  constexpr int n = S::n, n2 = S::n2, P = S::P, A = S::A, B = S::B, PL = S::PL;
+  __shared__ real su[S::ARR], sR[S::ARR], sS[S::ARR];
+  const int t = threadIdx.x;
+  const int le = t / n2, ij = t - le * n2;
+  const int64_t e = (int64_t)blockIdx.x * EPB + le;
+  const bool ok = le < EPB && e < E;
+  const int at = le * S::ES + ij % n + A * (ij / n);
+  const uint32_t lr = kHexLines<N, EPB, 1>.r[t], ls = kHexLines<N, EPB, 1>.s[t];
+  constexpr uint32_t kNone = HexLines<N, EPB, 1>::kNone;
+  real uc[n], g[n][6];
+  if (ok) {
+    int32_t node[n];
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      const int64_t ep = e * P + ij + n2 * k;
+      load_acoustic_rec<3>(rec, conn, ep, ep, g[k], &node[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < n; ++k) uc[k] = __ldg(u + node[k]);
+#pragma unroll
+    for (int k = 0; k < n; ++k) su[at + B * k] = uc[k];
+  }
+  __syncthreads();
+  if (lr != kNone) line_apply<n, 1, PL, false, 1>(su + lr, sR + lr, Dm);
+  if (ls != kNone) line_apply<n, A, PL, false, 1>(su + ls, sS + ls, Dm);
+  __syncthreads();
+  real o[n];
+  if (ok) {
+#pragma unroll
+    for (int k = 0; k < n; ++k) o[k] = 0;
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      const real dr = sR[at + B * k], ds = sS[at + B * k];
+      real dt = 0;
+#pragma unroll
+      for (int l = 0; l < n; ++l) dt += Dm.d[k * n + l] * uc[l];
+      // G00 G01 G02 G11 G12 G22
+      sR[at + B * k] = g[k][0] * dr + g[k][1] * ds + g[k][2] * dt;
+      sS[at + B * k] = g[k][1] * dr + g[k][3] * ds + g[k][4] * dt;
+      const real Ft = g[k][2] * dr + g[k][4] * ds + g[k][5] * dt;
+#pragma unroll
+      for (int m = 0; m < n; ++m) o[m] += Dm.d[k * n + m] * Ft;
+    }
+  }
+  __syncthreads();
+  if (lr != kNone) line_apply<n, 1, PL, true, 1>(sR + lr, sR + lr, Dm);
+  if (ls != kNone) line_apply<n, A, PL, true, 1>(sS + ls, sS + ls, Dm);
+  __syncthreads();
+  if (!ok) return;
+#pragma unroll
+  for (int k = 0; k < n; ++k)
+    r[e * P + ij + n2 * k] = -(o[k] + sR[at + B * k] + sS[at + B * k]);
 }
 
 }  // namespace salvus
