@@ -272,14 +272,15 @@ int salvus_problem_autotune(salvus_problem *p, int32_t *stiff_shot_lanes,
  *         stiffness kernel also advances each element's interior nodes; the
  *         gather covers the shared nodes only).  Both forms give bitwise the
  *         same fields.
- *   elements_per_cta  elements per CTA of the stiffness kernel where it is
- *         tuned (FP32 parallelepiped elastic hexahedra: 128 / (N+1)^2 or twice
- *         that; shot-batched quads: the batched kernel's elements), else 0.
- * FP32 single-shot elastic hexahedron meshes of parallelepipeds are tuned by
- * timing every admissible (form, CTA width) on scratch copies of the fields
- * before the first run (cached per mesh size and device for the process;
- * SALVUS_HEX_CONFIG="form,wide" pins the choice, SALVUS_HEX_STEP=fused or
- * plain forces the form).  Runs the tuning if it has not run yet. */
+ *   elements_per_cta  elements per CTA of the stiffness kernel (FP32
+ *         parallelepiped elastic hexahedra: 128 / (N+1)^2 or twice that;
+ *         shot-batched quads: the batched kernel's elements), else 0.
+ * FP32 single-shot elastic hexahedron meshes of parallelepipeds of orders 1-3
+ * are tuned by timing both CTA widths on scratch copies of the fields before
+ * the first run (cached per mesh size and device for the process); orders 4-6
+ * take the narrow one.  The fused form runs only where it is asked for
+ * (SALVUS_HEX_STEP=fused, or SALVUS_HEX_CONFIG="form,wide", which pins both).
+ * Runs the tuning if it has not run yet. */
 #define SALVUS_STEP_PLAIN 0
 #define SALVUS_STEP_FUSED_INTERIOR 1
 int salvus_problem_step_config(salvus_problem *p, int32_t *form, int32_t *elements_per_cta);
