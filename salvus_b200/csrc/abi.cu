@@ -240,9 +240,9 @@ static int acoustic2(const salvus_mesh *m, const real *rec, const real *u, real 
     const DMatrix<real> D = dmatrix<real>(m->basis);
     const int32_t *cn = m->d_conn.as<int32_t>();
     if constexpr (std::is_same<real, float>::value) {
-      if (m->qfactors) {
-        acoustic_quad_affine_kernel<N, EPB><<<blocks_for(m->E, EPB), S::THREADS, 0, s>>>(
-            m->E, m->d_qs32.as<float>(), m->d_qm32.as<float4>(), cn, u, r, D);
+      if (m->qscalar) {
+        acoustic_quad_square_kernel<N, EPB><<<blocks_for(m->E, EPB), S::THREADS, 0, s>>>(
+            m->E, m->d_qs32.as<float>(), cn, u, r, D);
         g_launches++;
         return check_launch("acoustic quad stiffness");
       }
@@ -586,7 +586,7 @@ static int build_records(salvus_mesh *m, DeviceBuffer &out, DeviceBuffer &mass_l
   geometry_kernel<real, kPack><<<blocks_for(total, 128), 128, 0, m->stream>>>(
       m->E, m->dim, m->n, m->P, m->physics, rw, m->d_vtx.as<double>(), m->d_par.as<double>(),
       m->d_conn.as<int32_t>(), gll, out.as<real>(), mass_local.as<double>(),
-      m->d_cls_k.as<int32_t>(), m->n_fluid, m->ti, m->qaffine);
+      m->d_cls_k.as<int32_t>(), m->n_fluid, m->ti, m->qsquare);
   g_launches++;
   return check_launch("geometry");
 }
@@ -733,19 +733,17 @@ static int mesh_setup_device(salvus_mesh *m) {
   } else if ((rc = build_records<float, true>(m, m->d_rec32, mass_local))) {
     return rc;
   }
-  if (m->qfactors) {
-    if ((rc = m->d_qs32.alloc(sizeof(float) * EP)) || (rc = m->d_qm32.alloc(sizeof(float4) * m->E)))
-      return rc;
+  if (m->qscalar) {
+    if ((rc = m->d_qs32.alloc(sizeof(float) * EP))) return rc;
     GllTable gll{};
     for (int i = 0; i < m->n; ++i) {
       gll.xi[i] = m->basis.xi[i];
       gll.w[i] = m->basis.w[i];
     }
-    quad_affine_factors_kernel<<<blocks_for(EP, 128), 128, 0, m->stream>>>(
-        m->E, m->n, m->P, m->d_vtx.as<double>(), m->d_par.as<double>(), gll, m->d_qs32.as<float>(),
-        m->d_qm32.as<float4>());
+    quad_square_kernel<<<blocks_for(EP, 128), 128, 0, m->stream>>>(
+        m->E, m->n, m->P, m->d_vtx.as<double>(), m->d_par.as<double>(), gll, m->d_qs32.as<float>());
     g_launches++;
-    if ((rc = check_launch("quad factors"))) return rc;
+    if ((rc = check_launch("squares"))) return rc;
   }
   // the node list of the fused steps (interior_free_nodes, at creation)
   if (m->n_gnodes > 0) {
@@ -1779,8 +1777,9 @@ static int group_fill(salvus_group *g) {
     int rc = ready(p);
     if (rc) return rc;
     GroupSlot &s = g->slots[k];
-    s.rec = m->qfactors ? m->d_qs32.as<float>() : m->d_rec32.as<float>();
-    s.jac = m->affine ? m->d_jac32.as<float>() : m->qfactors ? m->d_qm32.as<float>() : nullptr;
+    s.rec = m->qscalar ? m->d_qs32.as<float>() : m->d_rec32.as<float>();
+    s.jac = m->affine ? m->d_jac32.as<float>() : nullptr;
+    s.square = m->qscalar;
     s.conn = m->d_conn.as<int32_t>();
     s.inc_off = m->d_inc_off.as<int32_t>();
     s.inc_idx = m->d_inc_idx.as<int32_t>();
@@ -2207,19 +2206,20 @@ int salvus_mesh_create(const salvus_mesh_desc *d, int device, salvus_mesh **out)
     m->affine64 = affine && affine64;
   }
   if (m->shape == SALVUS_QUAD && m->physics != SALVUS_ELASTIC2D) {
-    // every element a parallelogram: opposite edges equal to 1e-9 of the
-    // shorter edge, which bounds how far the Jacobian varies over the element
-    // (FP32 rounds it at 6e-8)
-    bool para = true;
-    for (int64_t e = 0; e < m->E && para; ++e) {
+    // every element a square (opposite edges equal, adjacent ones equal and at a
+    // right angle) to 1e-10 of the edge: G then differs from a multiple of the
+    // identity by less than a hundredth of an FP32 rounding (6e-8)
+    m->qsquare = true;
+    for (int64_t e = 0; e < m->E && m->qsquare; ++e) {
       const double *v = m->vtx.data() + e * 8;
+      const double a[2] = {v[2] - v[0], v[3] - v[1]}, b[2] = {v[6] - v[0], v[7] - v[1]};
       const double off = std::hypot((v[0] - v[2]) + (v[4] - v[6]), (v[1] - v[3]) + (v[5] - v[7]));
-      const double a = std::hypot(v[2] - v[0], v[3] - v[1]), b = std::hypot(v[6] - v[0], v[7] - v[1]);
-      para = off <= 1e-9 * std::min(a, b);
+      const double aa = a[0] * a[0] + a[1] * a[1], bb = b[0] * b[0] + b[1] * b[1];
+      m->qsquare = off <= 1e-10 * std::sqrt(aa) && std::fabs(aa - bb) <= 1e-10 * aa &&
+                   std::fabs(a[0] * b[0] + a[1] * b[1]) <= 1e-10 * aa;
     }
-    m->qaffine = para;
-    m->qfactors = para && m->physics == SALVUS_ACOUSTIC &&
-                  !(d->reserved & SALVUS_MESH_PER_POINT_GEOMETRY);
+    m->qscalar = m->qsquare && m->physics == SALVUS_ACOUSTIC &&
+                 !(d->reserved & SALVUS_MESH_PER_POINT_GEOMETRY);
   }
   if ((rc = flatten_mesh(m.get(), d->cells, d->n_vertices))) return rc;
   if (m->physics == SALVUS_COUPLED2D && (rc = setup_coupled(m.get(), d->cells))) return rc;

@@ -142,11 +142,11 @@ struct salvus_mesh {
   // the same for FP64 (d_rec64, d_jac64): the Jacobians agree to the rounding
   // of the vertex coordinates
   bool affine64 = false;
-  // acoustic and fluid-solid quadrilaterals that are all parallelograms (FP32
-  // records then hold G as the product of its rounded factors); qfactors: the
-  // FP32 acoustic kernel reads the factors, d_qs32 [E][P] and d_qm32 [E] float4
-  bool qaffine = false, qfactors = false;
-  salvus::DeviceBuffer d_qs32, d_qm32;
+  // acoustic and fluid-solid quadrilaterals that are all squares: G is a
+  // multiple of the identity; qscalar: the FP32 single-shot acoustic kernel reads
+  // that number, d_qs32 [E][P], instead of the record
+  bool qsquare = false, qscalar = false;
+  salvus::DeviceBuffer d_qs32;
   // parallelepiped hexahedron kernels: CTAs of 128 / (N+1)^2 elements (0) or
   // twice that (1), set by the hexahedron autotuner
   int hex_wide = 0;

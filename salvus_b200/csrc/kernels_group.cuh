@@ -27,9 +27,10 @@ namespace salvus {
 
 struct GroupSlot {
   // mesh (jac != nullptr for meshes of parallelepipeds, whose rec holds the
-  // material planes of kernels_hex_affine.cuh, and of parallelograms, whose rec
-  // and jac are the factors of acoustic_quad_affine_kernel)
+  // material planes of kernels_hex_affine.cuh; square: a mesh of squares, whose
+  // rec holds the one number per point of acoustic_quad_square_kernel)
   const float *rec, *jac;
+  bool square;
   const int32_t *conn, *inc_off, *inc_idx;
   Incidence inc;  // quadrilaterals
   const float *mi;
@@ -69,9 +70,8 @@ template <int N>
 __device__ __forceinline__ void group_quad_body(const GroupSlot &m, int64_t bid,
                                                 const DMatrix<float> &Dm) {
   constexpr int EPB = quad_col_epb<N>();
-  if (m.jac)
-    acoustic_quad_col_body<N, EPB, float, 1, false, true>(
-        bid, m.E, m.rec, m.conn, m.u, m.r, Dm, nullptr, reinterpret_cast<const float4 *>(m.jac));
+  if (m.square)
+    acoustic_quad_col_body<N, EPB, float, 1, false, true>(bid, m.E, m.rec, m.conn, m.u, m.r, Dm);
   else
     acoustic_quad_col_body<N, EPB, float>(bid, m.E, m.rec, m.conn, m.u, m.r, Dm);
 }

@@ -37,18 +37,18 @@ struct QuadColShape {
 // Acoustic quads: r_e = -K_e u_e with G = w detJ vp^2 invJ^T invJ per point.
 // C / kList as in acoustic_stiffness_body (fluid elements of fluid-solid
 // meshes own component 0 of C and come from a list).
-// kAffine (FP32, every element a parallelogram): rec holds s = w detJ vp^2 per
-// point and met the element's metric; G = s metric is formed here (mul_rn: the
-// product the records hold, bit for bit).  8 instead of 16 bytes per point.
-template <int N, int EPB, typename real, int C = 1, bool kList = false, bool kAffine = false>
+// kSquare (FP32, every element a square): G is s times the identity and rec holds
+// s alone, 8 instead of 16 bytes per point with the node.  Other parallelograms
+// keep their records: s and an element's metric apart would be two more
+// roundings, one of them the same at every point of a uniform mesh.
+template <int N, int EPB, typename real, int C = 1, bool kList = false, bool kSquare = false>
 __device__ __forceinline__ void acoustic_quad_col_body(int64_t bid, int64_t nE,
                                                        const real *__restrict__ rec,
                                                        const int32_t *__restrict__ conn,
                                                        const real *__restrict__ u,
                                                        real *__restrict__ r,
                                                        const DMatrix<real> &Dm,
-                                                       const int32_t *__restrict__ elist = nullptr,
-                                                       const float4 *__restrict__ met = nullptr) {
+                                                       const int32_t *__restrict__ elist = nullptr) {
   using S = QuadColShape<N, EPB>;
   constexpr int n = S::n, P = S::P;
   __shared__ real sD[n * n];
@@ -66,7 +66,7 @@ __device__ __forceinline__ void acoustic_quad_col_body(int64_t bid, int64_t nE,
     int32_t node[n];
 #pragma unroll
     for (int j = 0; j < n; ++j) {
-      if constexpr (kAffine) {
+      if constexpr (kSquare) {
         node[j] = __ldg(conn + e * P + i + n * j);
         g0[j] = __ldg(rec + e * P + i + n * j);
       } else {
@@ -75,16 +75,6 @@ __device__ __forceinline__ void acoustic_quad_col_body(int64_t bid, int64_t nE,
         g0[j] = g[0];
         g1[j] = g[1];
         g2[j] = g[2];
-      }
-    }
-    if constexpr (kAffine) {
-      const float4 m = __ldg(met + e);
-#pragma unroll
-      for (int j = 0; j < n; ++j) {
-        const real s = g0[j];
-        g0[j] = mul_rn(s, m.x);
-        g1[j] = mul_rn(s, m.y);
-        g2[j] = mul_rn(s, m.z);
       }
     }
 #pragma unroll
@@ -110,8 +100,13 @@ __device__ __forceinline__ void acoustic_quad_col_body(int64_t bid, int64_t nE,
         gr += Dri[l] * su[le][l + n * j];
         gs += Dm.d[j * n + l] * uu[l];
       }
-      sF[le][i + n * j] = g0[j] * gr + g1[j] * gs;
-      Fs[j] = g1[j] * gr + g2[j] * gs;
+      if constexpr (kSquare) {
+        sF[le][i + n * j] = g0[j] * gr;
+        Fs[j] = g0[j] * gs;
+      } else {
+        sF[le][i + n * j] = g0[j] * gr + g1[j] * gs;
+        Fs[j] = g1[j] * gr + g2[j] * gs;
+      }
     }
   }
   __syncthreads();
@@ -141,11 +136,9 @@ acoustic_quad_col_kernel(int64_t E, const real *__restrict__ rec, const int32_t 
 
 template <int N, int EPB>
 __global__ void __launch_bounds__(QuadColShape<N, EPB>::THREADS)
-acoustic_quad_affine_kernel(int64_t E, const float *__restrict__ sq, const float4 *__restrict__ met,
-                            const int32_t *__restrict__ conn, const float *__restrict__ u,
-                            float *__restrict__ r, DMatrix<float> Dm) {
-  acoustic_quad_col_body<N, EPB, float, 1, false, true>(blockIdx.x, E, sq, conn, u, r, Dm, nullptr,
-                                                        met);
+acoustic_quad_square_kernel(int64_t E, const float *__restrict__ sq, const int32_t *__restrict__ conn,
+                            const float *__restrict__ u, float *__restrict__ r, DMatrix<float> Dm) {
+  acoustic_quad_col_body<N, EPB, float, 1, false, true>(blockIdx.x, E, sq, conn, u, r, Dm);
 }
 
 template <int N, int EPB, typename real>

@@ -87,41 +87,27 @@ __device__ __forceinline__ double p1_interp_dev(int dim, const double *vals, con
   return s;
 }
 
-// Parallelogram quadrilaterals: the metric sum_x invJ[x][a] invJ[x][b] of an
-// element (at its centre), and G = s metric as the single-shot kernel forms it
-// from the stored factors -- one rounded product of two FP32 values -- so that
-// records and factors give the same bits.
-__device__ __forceinline__ void quad_metric(const double *v, double *m) {
-  const double c0[3] = {0.0, 0.0, 0.0};
-  double d0, J[4];
-  p1_jac_dev(2, v, c0, &d0, J);
-  m[0] = J[0] * J[0] + J[2] * J[2];
-  m[1] = J[0] * J[1] + J[2] * J[3];
-  m[2] = J[1] * J[1] + J[3] * J[3];
+// Meshes of squares (salvus_mesh::qsquare): G = g I with g = w detJ vp^2 times the
+// metric's diagonal, formed in FP64 and rounded once, in the records as in the
+// layout that keeps g alone, so that both give the same bits.
+__device__ __forceinline__ float quad_square_g(double s, const double *iJ) {
+  return (float)(s * (0.5 * (iJ[0] * iJ[0] + iJ[2] * iJ[2] + iJ[1] * iJ[1] + iJ[3] * iJ[3])));
 }
-__device__ __forceinline__ void quad_affine_metric(const double *v, double s, float *g) {
-  double m[3];
-  quad_metric(v, m);
-  for (int a = 0; a < 3; ++a) g[a] = __fmul_rn((float)s, (float)m[a]);
-}
-__global__ void quad_affine_factors_kernel(int64_t E, int n, int P, const double *__restrict__ vtx,
-                                           const double *__restrict__ par, GllTable gll,
-                                           float *__restrict__ sq, float4 *__restrict__ met) {
+__global__ void quad_square_kernel(int64_t E, int n, int P, const double *__restrict__ vtx,
+                                   const double *__restrict__ par, GllTable gll,
+                                   float *__restrict__ sq) {
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= E * P) return;
   const int64_t e = tid / P;
   const int p = (int)(tid - e * P);
   const double ref[3] = {gll.xi[p % n], gll.xi[p / n], 0.0};
-  double v[8], vals[4], detJ, iJ[4], m[3];
+  double v[8], vals[4], detJ, iJ[4];
   for (int a = 0; a < 8; ++a) v[a] = vtx[e * 8 + a];
   for (int a = 0; a < 4; ++a) vals[a] = par[e * 4 + a];
   p1_jac_dev(2, v, ref, &detJ, iJ);
-  const double vp = p1_interp_dev(2, vals, ref);
-  sq[tid] = (float)(gll.w[p % n] * gll.w[p / n] * 1.0 * detJ * vp * vp);
-  if (p == 0) {
-    quad_metric(v, m);
-    met[e] = make_float4((float)m[0], (float)m[1], (float)m[2], 0.f);
-  }
+  const double wq = gll.w[p % n] * gll.w[p / n] * 1.0;
+  const double wd = wq * detJ, vp = p1_interp_dev(2, vals, ref);
+  sq[tid] = quad_square_g(wd * vp * vp, iJ);
 }
 
 // One thread per element point.  Writes the stiffness record (FP32 packed
@@ -144,7 +130,7 @@ __global__ void geometry_kernel(int64_t E, int dim, int n, int P, int physics, i
                                 const int32_t *__restrict__ conn, GllTable gll,
                                 real *__restrict__ rec, double *__restrict__ mass_local,
                                 const int32_t *__restrict__ cls_k = nullptr, int64_t Ef = 0,
-                                bool ti = false, bool qaffine = false) {
+                                bool ti = false, bool qsquare = false) {
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= E * P) return;
   const int64_t e = tid / P;
@@ -175,7 +161,7 @@ __global__ void geometry_kernel(int64_t E, int dim, int n, int P, int physics, i
       if constexpr (kPackConn) {
         real *o = rec + (k * P + p) * 4;
         for (int a = 0; a < 3; ++a) o[a] = (real)g3[a];
-        if (qaffine) quad_affine_metric(v, sc, o);
+        if (qsquare) o[0] = o[2] = quad_square_g(sc, iJ), o[1] = 0;
         reinterpret_cast<int32_t *>(o)[3] = conn[tid];
       } else {
         real *o = rec + (k * P + p) * 3;
@@ -225,7 +211,7 @@ __global__ void geometry_kernel(int64_t E, int dim, int n, int P, int physics, i
       double g11 = iJ[1] * iJ[1] + iJ[3] * iJ[3];
       out[0] = (real)(s * g00); out[1] = (real)(s * g01); out[2] = (real)(s * g11);
       if constexpr (kPackConn) {
-        if (qaffine) quad_affine_metric(v, s, out);
+        if (qsquare) out[0] = out[2] = quad_square_g(s, iJ), out[1] = 0;
       }
     } else {
       int q = 0;
