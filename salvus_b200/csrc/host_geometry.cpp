@@ -231,6 +231,20 @@ void p1_jacobian(int shape, const double *vtx, const double *ref, double *detJ, 
   inverse3(J, detJ, invJ);
 }
 
+void p1_jacobian_edges(const double *vtx, double *detJ, double *invJ) {
+  static const int ends[3][4][2] = {{{0, 3}, {1, 2}, {4, 5}, {7, 6}},
+                                    {{0, 1}, {3, 2}, {4, 7}, {5, 6}},
+                                    {{0, 4}, {1, 7}, {2, 6}, {3, 5}}};
+  double J[9];
+  for (int k = 0; k < 3; ++k)
+    for (int m = 0; m < 3; ++m) {
+      double d[4];
+      for (int q = 0; q < 4; ++q) d[q] = vtx[3 * ends[k][q][1] + m] - vtx[3 * ends[k][q][0] + m];
+      J[3 * k + m] = 0.125 * ((d[0] + d[1]) + (d[2] + d[3]));
+    }
+  inverse3(J, detJ, invJ);
+}
+
 static void inverse3(const double *J, double *detJ, double *invJ) {
   double m00 = J[4] * J[8] - J[5] * J[7], m01 = J[5] * J[6] - J[3] * J[8],
          m02 = J[3] * J[7] - J[4] * J[6];

@@ -54,6 +54,12 @@ double point_weight(const Basis &b, int p);
 // P1 geometry of one element: vertex signs of QuadP1.h:98-108 / HexP1.cpp,
 // affine maps of TriP1.cpp:56-94 / TetP1.cpp:91-150.
 void p1_jacobian(int shape, const double *vtx, const double *ref, double *detJ, double *invJ);
+// The same of a hexahedron that is a parallelepiped, each row the mean of its
+// four edges.  The edges are subtracted before anything is added, so the result
+// carries the rounding of the coordinates only, not that of sums of coordinates:
+// rms error at the GLL points against extended precision 0.02 to 0.8 times that
+// of p1_jacobian there on boxes at offsets up to 10^5.
+void p1_jacobian_edges(const double *vtx, double *detJ, double *invJ);
 void p1_map(int shape, const double *vtx, const double *ref, double *x);
 void p1_weights(int shape, const double *ref, double *w);  // vertex weights [nv]
 int check_hull(int shape, const double *vtx, const double *x);  // 1 in, 0 out, <0 error
@@ -140,7 +146,7 @@ struct salvus_mesh {
   // the nodes that are not interior to an element (fused steps' gather)
   bool affine = false;
   // the same for FP64 (d_rec64, d_jac64): the Jacobians agree to the rounding
-  // of the vertex coordinates
+  // of the sums that form a point's own (eps |x| / 2h)
   bool affine64 = false;
   // acoustic and fluid-solid quadrilaterals that are all squares: G is a
   // multiple of the identity; qscalar: the FP32 single-shot acoustic kernel reads

@@ -24,6 +24,23 @@ struct GllTable {
   double w[kMaxN];
 };
 
+__device__ __forceinline__ void inverse3_dev(const double *J, double *detJ, double *invJ) {
+  double m00 = J[4] * J[8] - J[5] * J[7], m01 = J[5] * J[6] - J[3] * J[8],
+         m02 = J[3] * J[7] - J[4] * J[6];
+  double d = J[0] * m00 + J[1] * m01 + J[2] * m02;
+  double id = 1.0 / d;
+  *detJ = d;
+  invJ[0] = m00 * id;
+  invJ[1] = (J[2] * J[7] - J[1] * J[8]) * id;
+  invJ[2] = (J[1] * J[5] - J[2] * J[4]) * id;
+  invJ[3] = m01 * id;
+  invJ[4] = (J[0] * J[8] - J[2] * J[6]) * id;
+  invJ[5] = (J[2] * J[3] - J[0] * J[5]) * id;
+  invJ[6] = m02 * id;
+  invJ[7] = (J[1] * J[6] - J[0] * J[7]) * id;
+  invJ[8] = (J[0] * J[4] - J[1] * J[3]) * id;
+}
+
 __device__ __forceinline__ void p1_jac_dev(int dim, const double *v, const double *ref,
                                            double *detJ, double *invJ) {
   if (dim == 2) {
@@ -56,20 +73,26 @@ __device__ __forceinline__ void p1_jac_dev(int dim, const double *v, const doubl
       J[6 + m] += d2 * v[3 * k + m];
     }
   }
-  double m00 = J[4] * J[8] - J[5] * J[7], m01 = J[5] * J[6] - J[3] * J[8],
-         m02 = J[3] * J[7] - J[4] * J[6];
-  double d = J[0] * m00 + J[1] * m01 + J[2] * m02;
-  double id = 1.0 / d;
-  *detJ = d;
-  invJ[0] = m00 * id;
-  invJ[1] = (J[2] * J[7] - J[1] * J[8]) * id;
-  invJ[2] = (J[1] * J[5] - J[2] * J[4]) * id;
-  invJ[3] = m01 * id;
-  invJ[4] = (J[0] * J[8] - J[2] * J[6]) * id;
-  invJ[5] = (J[2] * J[3] - J[0] * J[5]) * id;
-  invJ[6] = m02 * id;
-  invJ[7] = (J[1] * J[6] - J[0] * J[7]) * id;
-  invJ[8] = (J[0] * J[4] - J[1] * J[3]) * id;
+  inverse3_dev(J, detJ, invJ);
+}
+
+// Inverse Jacobian of a parallelepiped: each row the mean of its four edges,
+// the edges subtracted first (p1_jacobian_edges on the host).
+__device__ __forceinline__ void edge_jac_dev(const double *v, double *invJ) {
+  const int ends[3][4][2] = {{{0, 3}, {1, 2}, {4, 5}, {7, 6}},
+                             {{0, 1}, {3, 2}, {4, 7}, {5, 6}},
+                             {{0, 4}, {1, 7}, {2, 6}, {3, 5}}};
+  double J[9], detJ;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      double d[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) d[q] = v[3 * ends[k][q][1] + m] - v[3 * ends[k][q][0] + m];
+      J[3 * k + m] = 0.125 * ((d[0] + d[1]) + (d[2] + d[3]));
+    }
+  inverse3_dev(J, &detJ, invJ);
 }
 
 __device__ __forceinline__ double p1_interp_dev(int dim, const double *vals, const double *ref) {
@@ -269,8 +292,8 @@ __global__ void geometry_kernel(int64_t E, int dim, int n, int P, int physics, i
 // (kernels_hex_affine.cuh): one thread per element point writes the folded
 // material planes mat[m][e*P + p] (w detJ at the point times the constants
 // of the P1-interpolated parameters, as geometry_kernel) and the
-// element-local mass; point 0 of each element also writes invJ at the
-// element centre to jac[e][9] (constant over an affine element).
+// element-local mass; point 0 of each element also writes the element's invJ
+// (edge_jac_dev) to jac[e][9].
 template <typename real>
 __global__ void affine_hex_records_kernel(int64_t E, int n, int P, bool ti,
                                           const double *__restrict__ vtx,
@@ -303,9 +326,8 @@ __global__ void affine_hex_records_kernel(int64_t E, int n, int P, bool ti,
   for (int q = 0; q < nm; ++q) mat[(int64_t)q * E * P + tid] = (real)(wd * mc[q]);
   mass_local[tid] = wd * pv[0];
   if (p == 0) {
-    const double c0[3] = {0.0, 0.0, 0.0};
-    double d0, J0[9];
-    p1_jac_dev(3, v, c0, &d0, J0);
+    double J0[9];
+    edge_jac_dev(v, J0);
     for (int a = 0; a < 9; ++a) jac[e * 9 + a] = (real)J0[a];
   }
 }
