@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "once_per_device.h"
 #include "kernels_setup.cuh"
 #include "kernels_stiffness.cuh"
 #include "kernels_step.cuh"
@@ -119,17 +120,25 @@ static bool hex_classic() {
   return s && std::strcmp(s, "classic") == 0;
 }
 
+// Lets a kernel's launches on the mesh's device, which is the current one, use
+// `bytes` of dynamic shared memory (more than 48 KB has to be asked for).
+template <typename Kern>
+static int dynamic_smem(OncePerDevice &once, const salvus_mesh *m, Kern kern, size_t bytes) {
+  const int e = once(m->device, [&] {
+    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  });
+  if (e == 0) return SALVUS_OK;
+  return fail(SALVUS_E_CUDA, "%zu bytes of shared memory refused: %s", bytes,
+              cudaGetErrorString((cudaError_t)e));
+}
+
 template <int N, bool TI>
 static int launch_elastic_v2(const salvus_mesh *m, const float *rec, const float *u, float *r,
                              cudaStream_t st) {
   constexpr int n2 = (N + 1) * (N + 1), EPB = 128 / n2 > 0 ? 128 / n2 : 1;
   using T = ElasticV2Shape<N, EPB, TI>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(elastic_hex_stiffness_v2_kernel<N, EPB, TI>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
-    attr = true;
-  }
+  static OncePerDevice attr;
+  if (int rc = dynamic_smem(attr, m, elastic_hex_stiffness_v2_kernel<N, EPB, TI>, T::SMEM)) return rc;
   elastic_hex_stiffness_v2_kernel<N, EPB, TI><<<blocks_for(m->E, EPB), T::THREADS, T::SMEM, st>>>(
       m->E, rec, u, r, dmatrix<float>(m->basis));
   g_launches++;
@@ -140,12 +149,8 @@ template <int N, typename real, bool TI>
 static int launch_elastic_classic(const salvus_mesh *m, const real *rec, const real *u, real *r,
                                   cudaStream_t st) {
   using S = ElasticShape<N, real>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(elastic_hex_stiffness_kernel<N, real, TI>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    attr_set = true;
-  }
+  static OncePerDevice attr;
+  if (int rc = dynamic_smem(attr, m, elastic_hex_stiffness_kernel<N, real, TI>, S::SMEM)) return rc;
   elastic_hex_stiffness_kernel<N, real, TI><<<blocks_for(m->E, S::EPB), S::THREADS, S::SMEM, st>>>(
       m->E, rec, m->d_conn.as<int32_t>(), u, r, dmatrix<real>(m->basis));
   g_launches++;
@@ -162,11 +167,8 @@ static int launch_elastic_affine_epb(const salvus_mesh *m, const float *mat, flo
   using T = HexAffineShape<N, EPB, TI>;
   auto kern = kFuse ? elastic_hex_affine_fused_kernel<N, EPB, TI>
                     : elastic_hex_affine_kernel<N, EPB, TI>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
-    attr = true;
-  }
+  static OncePerDevice attr;
+  if (int rc = dynamic_smem(attr, m, kern, T::SMEM)) return rc;
   kern<<<blocks_for(m->E, EPB), T::THREADS, T::SMEM, st>>>(
       m->E, m->d_jac32.as<float>(), mat, m->d_conn.as<int32_t>(), u, r, dmatrix<float>(m->basis),
       iu);
@@ -186,12 +188,8 @@ static int launch_elastic_col64(const salvus_mesh *m, const double *rec, const d
                                 cudaStream_t st) {
   constexpr int EPB = HexCol64<N, TI, kAffine>::EPB;
   using T = HexColShape<N, EPB, double>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(elastic_hex_col64_kernel<N, TI, kAffine>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
-    attr = true;
-  }
+  static OncePerDevice attr;
+  if (int rc = dynamic_smem(attr, m, elastic_hex_col64_kernel<N, TI, kAffine>, T::SMEM)) return rc;
   elastic_hex_col64_kernel<N, TI, kAffine><<<blocks_for(m->E, EPB), T::THREADS, T::SMEM, st>>>(
       m->E, m->d_jac64.as<double>(), rec, m->d_conn.as<int32_t>(), const_cast<double *>(u), r,
       dmatrix<double>(m->basis));
@@ -348,12 +346,8 @@ template <typename real, int C, bool TI = false>
 static int launch_tet(const salvus_mesh *m, const real *rec, const real *u, real *r,
                       cudaStream_t st) {
   using S = TetShape<real, C, TI>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(tet_stiffness_kernel<real, C, TI>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
-    attr = true;
-  }
+  static OncePerDevice attr;
+  if (int rc = dynamic_smem(attr, m, tet_stiffness_kernel<real, C, TI>, S::SMEM)) return rc;
   tet_stiffness_kernel<real, C, TI><<<blocks_for(m->E, S::EPB), S::THREADS, S::SMEM, st>>>(
       m->E, rec, m->d_conn.as<int32_t>(), simplex_tables<real>(m), u, r);
   g_launches++;
@@ -365,12 +359,8 @@ template <int C>
 static int launch_tet_tc(const salvus_mesh *m, const float *rec, const float *u, float *r,
                          cudaStream_t st, int *err, long long wlim, int hold) {
   using S = TetTcShape<C>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(tet_tc_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)S::SMEM);
-    attr = true;
-  }
+  static OncePerDevice attr;
+  if (int rc = dynamic_smem(attr, m, tet_tc_kernel<C>, S::SMEM)) return rc;
   const int64_t tiles = (m->E + S::NE - 1) / S::NE;
   const unsigned grid = (unsigned)(tiles < m->sm_count ? tiles : m->sm_count);
   tet_tc_kernel<C><<<grid, S::THREADS, S::SMEM, st>>>(
@@ -382,12 +372,15 @@ static int launch_tet_tc(const salvus_mesh *m, const float *rec, const float *u,
 static int launch_tri_tc(const salvus_mesh *m, const float *rec, const float *u, float *r,
                          cudaStream_t st, int *err, long long wlim, int hold) {
   using S = TriTcShape;
-  static int per_sm = 0;
-  if (!per_sm) {
-    cudaFuncSetAttribute(tri_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+  static OncePerDevice attr;
+  if (int rc = dynamic_smem(attr, m, tri_tc_kernel, S::SMEM)) return rc;
+  static std::atomic<int> resident{0};  // CTAs per SM, the same on every device this runs on
+  int per_sm = resident.load();
+  if (per_sm == 0) {
     SALVUS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tri_tc_kernel, S::THREADS,
                                                               S::SMEM));
     if (per_sm < 1) per_sm = 1;
+    resident = per_sm;
   }
   const int64_t tiles = (m->E + S::NE - 1) / S::NE;
   const int64_t slots = (int64_t)per_sm * m->sm_count;
@@ -1679,12 +1672,8 @@ static int group_stiffness_t(const salvus_mesh *m0, const GroupSlot *slots, cons
   } else if constexpr (N <= kMaxHexOrder) {
     constexpr int n2 = (N + 1) * (N + 1), EPB = 128 / n2 > 0 ? 128 / n2 : 1;
     using T = ElasticV2Shape<N, EPB, false>;
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(group_hex_elastic_stiffness<N, EPB>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
-      attr = true;
-    }
+    static OncePerDevice attr;
+    if (int rc = dynamic_smem(attr, m0, group_hex_elastic_stiffness<N, EPB>, T::SMEM)) return rc;
     group_hex_elastic_stiffness<N, EPB><<<(unsigned)blocks, T::THREADS, T::SMEM, st>>>(
         slots, owner, dmatrix<float>(m0->basis));
   }
@@ -1881,7 +1870,7 @@ static int group_persistent_t(salvus_group *g, bool store_a) {
   }
   auto kern = group_persistent_step<N, kHex, C>;
   if (g->grid == 0) {
-    if (smem) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem) SALVUS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     SALVUS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
     g->grid = (per_sm > 0 ? per_sm : 1) * g->m0->sm_count;
