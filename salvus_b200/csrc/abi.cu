@@ -1128,11 +1128,14 @@ static int step_fused_t(salvus_problem *p, bool store_a) {
 // shot-batched step (FP32 acoustic quads)
 struct BatchCfg {
   int sc, epc, npt;  // shots, elements / node groups per CTA, nodes per thread
+  bool timed = false;  // a candidate of the autotuner; the others run where they are pinned
 };
-// Stiffness: the third number is the shots per thread; {0, 1, 2} takes CTAs of
-// pair_shots.  Below 64 shots its CTAs would be less than a warp.
-static const BatchCfg kStiffCfg[] = {{32, 1, 1}, {32, 2, 1}, {32, 4, 1}, {64, 1, 1},
-                                     {128, 1, 1}, {0, 1, 2}};
+// The places in these lists are what SALVUS_BATCH_CONFIG names: new shapes go to
+// the end.  Stiffness: the third number is the shots per thread; {0, 1, 2} takes
+// CTAs of pair_shots.  Below 64 shots its CTAs would be less than a warp.
+static const BatchCfg kStiffCfg[] = {{32, 1, 1, true}, {32, 2, 1, true}, {32, 4, 1, true},
+                                     {64, 1, 1, true}, {64, 2, 1},       {128, 1, 1, true},
+                                     {128, 2, 1},      {256, 1, 1},      {0, 1, 2, true}};
 // shots per CTA of {0, 1, 2}: the most 32-shot groups, up to eight, that
 // divide the padded shots
 static int pair_shots(int shots_pad) {
@@ -1144,9 +1147,15 @@ static bool stiff_cfg_fits(int cfg, int shots_pad) {
   const int sc = kStiffCfg[cfg].sc;
   return sc ? shots_pad % sc == 0 : pair_shots(shots_pad) >= 64;
 }
-static const BatchCfg kGatherCfg[] = {{32, 16, 1}, {32, 32, 1}, {64, 8, 1}, {64, 16, 1},
-                                      {128, 4, 1}, {128, 8, 1}, {256, 2, 1}, {256, 4, 1},
-                                      {32, 16, 2}, {64, 8, 2},  {128, 4, 2}, {256, 2, 2}};
+// Gather: 32 to 64 threads in the first twelve (four shots a thread), 128 to 256
+// in the others, which the autotuner times.
+static const BatchCfg kGatherCfg[] = {
+    {32, 4, 1},         {32, 8, 1},         {64, 2, 1},         {64, 4, 1},
+    {128, 1, 1},        {128, 2, 1},        {256, 1, 1},        {32, 4, 2},
+    {64, 2, 2},         {128, 1, 2},        {128, 1, 4},        {256, 1, 2},
+    {32, 16, 1, true},  {32, 32, 1, true},  {64, 8, 1, true},   {64, 16, 1, true},
+    {128, 4, 1, true},  {128, 8, 1, true},  {256, 2, 1, true},  {256, 4, 1, true},
+    {32, 16, 2, true},  {64, 8, 2, true},   {128, 4, 2, true},  {256, 2, 2, true}};
 constexpr int kNumStiffCfg = sizeof(kStiffCfg) / sizeof(kStiffCfg[0]);
 constexpr int kNumGatherCfg = sizeof(kGatherCfg) / sizeof(kGatherCfg[0]);
 
@@ -1190,8 +1199,11 @@ static int launch_qb_cfg(const salvus_problem *p, int cfg, cudaStream_t st, bool
     case 1: launch_qb<N, 32, 2, 1>(p, st, fuse); break;
     case 2: launch_qb<N, 32, 4, 1>(p, st, fuse); break;
     case 3: launch_qb<N, 64, 1, 1>(p, st, fuse); break;
-    case 4: launch_qb<N, 128, 1, 1>(p, st, fuse); break;
-    case 5: launch_qb<N, 0, 1, 2>(p, st, fuse); break;
+    case 4: launch_qb<N, 64, 2, 1>(p, st, fuse); break;
+    case 5: launch_qb<N, 128, 1, 1>(p, st, fuse); break;
+    case 6: launch_qb<N, 128, 2, 1>(p, st, fuse); break;
+    case 7: launch_qb<N, 256, 1, 1>(p, st, fuse); break;
+    case 8: launch_qb<N, 0, 1, 2>(p, st, fuse); break;
     default: return fail(SALVUS_E_INVALID, "bad batch config %d", cfg);
   }
   g_launches++;
@@ -1225,18 +1237,30 @@ static void launch_bg(const salvus_problem *p, cudaStream_t st, bool fuse, int64
 static int batched_gather(const salvus_problem *p, int cfg, cudaStream_t st, bool fuse,
                           int64_t *step) {
   switch (cfg) {
-    case 0: launch_bg<32, 16>(p, st, fuse, step); break;
-    case 1: launch_bg<32, 32>(p, st, fuse, step); break;
-    case 2: launch_bg<64, 8>(p, st, fuse, step); break;
-    case 3: launch_bg<64, 16>(p, st, fuse, step); break;
-    case 4: launch_bg<128, 4>(p, st, fuse, step); break;
-    case 5: launch_bg<128, 8>(p, st, fuse, step); break;
-    case 6: launch_bg<256, 2>(p, st, fuse, step); break;
-    case 7: launch_bg<256, 4>(p, st, fuse, step); break;
-    case 8: launch_bg<32, 16, 2>(p, st, fuse, step); break;
-    case 9: launch_bg<64, 8, 2>(p, st, fuse, step); break;
-    case 10: launch_bg<128, 4, 2>(p, st, fuse, step); break;
-    case 11: launch_bg<256, 2, 2>(p, st, fuse, step); break;
+    case 0: launch_bg<32, 4>(p, st, fuse, step); break;
+    case 1: launch_bg<32, 8>(p, st, fuse, step); break;
+    case 2: launch_bg<64, 2>(p, st, fuse, step); break;
+    case 3: launch_bg<64, 4>(p, st, fuse, step); break;
+    case 4: launch_bg<128, 1>(p, st, fuse, step); break;
+    case 5: launch_bg<128, 2>(p, st, fuse, step); break;
+    case 6: launch_bg<256, 1>(p, st, fuse, step); break;
+    case 7: launch_bg<32, 4, 2>(p, st, fuse, step); break;
+    case 8: launch_bg<64, 2, 2>(p, st, fuse, step); break;
+    case 9: launch_bg<128, 1, 2>(p, st, fuse, step); break;
+    case 10: launch_bg<128, 1, 4>(p, st, fuse, step); break;
+    case 11: launch_bg<256, 1, 2>(p, st, fuse, step); break;
+    case 12: launch_bg<32, 16>(p, st, fuse, step); break;
+    case 13: launch_bg<32, 32>(p, st, fuse, step); break;
+    case 14: launch_bg<64, 8>(p, st, fuse, step); break;
+    case 15: launch_bg<64, 16>(p, st, fuse, step); break;
+    case 16: launch_bg<128, 4>(p, st, fuse, step); break;
+    case 17: launch_bg<128, 8>(p, st, fuse, step); break;
+    case 18: launch_bg<256, 2>(p, st, fuse, step); break;
+    case 19: launch_bg<256, 4>(p, st, fuse, step); break;
+    case 20: launch_bg<32, 16, 2>(p, st, fuse, step); break;
+    case 21: launch_bg<64, 8, 2>(p, st, fuse, step); break;
+    case 22: launch_bg<128, 4, 2>(p, st, fuse, step); break;
+    case 23: launch_bg<256, 2, 2>(p, st, fuse, step); break;
     default: return fail(SALVUS_E_INVALID, "bad gather config %d", cfg);
   }
   g_launches++;
@@ -1308,14 +1332,14 @@ static int autotune(salvus_problem *p) {
     cudaMemsetAsync(p->d_u.ptr, 0, nf, p->stream);
     cudaMemsetAsync(p->d_v.ptr, 0, nf, p->stream);
     for (int c = 0; c < kNumStiffCfg && rc == SALVUS_OK; ++c) {
-      if (!stiff_cfg_fits(c, p->shots_pad)) continue;
+      if (!kStiffCfg[c].timed || !stiff_cfg_fits(c, p->shots_pad)) continue;
       float t = time_it([&] { return batched_stiffness(p, c, p->stream, fuse); });
       if (t < bs) { bs = t; cs = c; }
     }
     float bg = 1e30f;
     int cg = -1;
     for (int c = 0; c < kNumGatherCfg && rc == SALVUS_OK; ++c) {
-      if (p->shots_pad % kGatherCfg[c].sc) continue;
+      if (!kGatherCfg[c].timed || p->shots_pad % kGatherCfg[c].sc) continue;
       float t = time_it([&] { return batched_gather(p, c, p->stream, fuse, nullptr); });
       if (t < bg) { bg = t; cg = c; }
     }
