@@ -260,8 +260,9 @@ int64_t salvus_problem_step_index(const salvus_problem *p);
  * kernel and the shot lanes and nodes per CTA of the batched gather/update
  * (no reference counterpart; the reference runs one source set per run).
  * Runs automatically before the first batched step; results are cached per
- * (order, shots, elements, device).  Single-shot problems report fixed
- * values.  SALVUS_BATCH_CONFIG="i,j" pins the choice. */
+ * (order, shots, elements, device, step form).  Single-shot problems report
+ * fixed values.  SALVUS_BATCH_CONFIG="i,j" in the environment, where the shapes
+ * that the indices name fit the shots, pins the choice and is not cached. */
 int salvus_problem_autotune(salvus_problem *p, int32_t *stiff_shot_lanes,
                             int32_t *stiff_elements, int32_t *gather_shot_lanes,
                             int32_t *gather_nodes);

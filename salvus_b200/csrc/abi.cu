@@ -1271,27 +1271,12 @@ static int batched_gather(const salvus_problem *p, int cfg, cudaStream_t st, boo
 // kernels on this problem and keeps the fastest.  The stiffness timing writes
 // only the residual scratch; the gather timing runs on copies of u and w, so
 // the problem's state is untouched.  Results are cached per (order, padded
-// shots, elements, device) for the process.
+// shots, elements, device, step form) for the process.
 static int autotune(salvus_problem *p) {
   if (p->tune_stiff >= 0 && p->tune_gather >= 0) return SALVUS_OK;
-  struct Key {
-    int order, shots;
-    int64_t E;
-    int dev;
-  };
-  static std::mutex cache_mu;
-  static std::vector<std::pair<Key, std::pair<int, int>>> cache;
-  {
-    std::lock_guard<std::mutex> lk(cache_mu);
-    for (auto &c : cache)
-      if (c.first.order == p->mesh->order && c.first.shots == p->shots_pad &&
-          c.first.E == p->mesh->E && c.first.dev == p->mesh->device) {
-        p->tune_stiff = c.second.first;
-        p->tune_gather = c.second.second;
-        return SALVUS_OK;
-      }
-  }
-  const char *env = std::getenv("SALVUS_BATCH_CONFIG");  // "stiff,gather" fixes the choice
+  // "stiff,gather" fixes the choice, whatever other problems of this size were
+  // tuned to
+  const char *env = std::getenv("SALVUS_BATCH_CONFIG");
   if (env) {
     int a = -1, b = -1;
     if (std::sscanf(env, "%d,%d", &a, &b) == 2 && a >= 0 && a < kNumStiffCfg && b >= 0 &&
@@ -1300,6 +1285,25 @@ static int autotune(salvus_problem *p) {
       p->tune_gather = b;
       return SALVUS_OK;
     }
+  }
+  struct Key {
+    int order, shots;
+    int64_t E;
+    int dev;
+    bool fuse;  // the two forms of the step move different work
+  };
+  const bool fuse = batch_fusion(p);
+  static std::mutex cache_mu;
+  static std::vector<std::pair<Key, std::pair<int, int>>> cache;
+  {
+    std::lock_guard<std::mutex> lk(cache_mu);
+    for (auto &c : cache)
+      if (c.first.order == p->mesh->order && c.first.shots == p->shots_pad &&
+          c.first.E == p->mesh->E && c.first.dev == p->mesh->device && c.first.fuse == fuse) {
+        p->tune_stiff = c.second.first;
+        p->tune_gather = c.second.second;
+        return SALVUS_OK;
+      }
   }
   cudaEvent_t e0, e1;
   SALVUS_CUDA(cudaEventCreate(&e0));
@@ -1321,7 +1325,6 @@ static int autotune(salvus_problem *p) {
   // both kernels are timed on zeroed scratch copies of u and w (the fused
   // stiffness kernel also advances interior nodes), so the problem's state
   // is untouched
-  const bool fuse = batch_fusion(p);
   const size_t nf = (size_t)p->mesh->G * p->shots_pad * sizeof(float);
   DeviceBuffer su, sw;
   float bs = 1e30f;
@@ -1354,7 +1357,7 @@ static int autotune(salvus_problem *p) {
   if (cs < 0 || p->tune_gather < 0) return fail(SALVUS_E_INVALID, "no admissible batch configuration");
   p->tune_stiff = cs;
   std::lock_guard<std::mutex> lk(cache_mu);
-  cache.push_back({{p->mesh->order, p->shots_pad, p->mesh->E, p->mesh->device},
+  cache.push_back({{p->mesh->order, p->shots_pad, p->mesh->E, p->mesh->device, fuse},
                    {p->tune_stiff, p->tune_gather}});
   return SALVUS_OK;
 }

@@ -1,5 +1,7 @@
 """SALVUS_BATCH_CONFIG="i,j": the CTA shapes that the indices stand for, read
-back from salvus_problem_autotune, and their results, which are the same bits."""
+back from salvus_problem_autotune, their results, which are the same
+bits, and that a pin holds after other problems of the same size have been
+tuned."""
 import numpy as np
 import pytest
 
@@ -49,3 +51,17 @@ def test_indices_pin_their_shapes(order, step, monkeypatch):
         assert np.abs(want[1]).max() > 0
         for a, b in zip(got, want):
             assert np.array_equal(a, b), (i, j)
+
+
+def test_pin_after_tuning(monkeypatch):
+    """Tuning results are shared by problems of one size; a pin is not lost to them."""
+    cfg = configs.batched_quad(nel=7, order=3, n_shots=64, n_receivers=1)
+    mesh = core.Mesh(cfg["shape"], cfg["order"], cfg["physics"], cfg["vertices"], cfg["cells"],
+                     cfg["params"])
+    monkeypatch.delenv("SALVUS_BATCH_CONFIG", raising=False)
+    tuned = problem(mesh, cfg, 64).autotune()
+    for i, j in ((0, 0), (1, 3), (2, 1)):
+        monkeypatch.setenv("SALVUS_BATCH_CONFIG", f"{i},{j}")
+        assert problem(mesh, cfg, 64).autotune() == (*STIFFNESS[i], *GATHER[j])
+    monkeypatch.setenv("SALVUS_BATCH_CONFIG", "5,0")  # 128 shots per CTA: not at 64 shots
+    assert problem(mesh, cfg, 64).autotune() == tuned
