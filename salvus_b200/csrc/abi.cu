@@ -2782,22 +2782,26 @@ int salvus_problem_get_field(salvus_problem *p, int32_t f, int32_t shot, double 
     if (rc) return rc;
   } else {
     int rc;
-    if (p->d_stage.bytes < 8 * N && (rc = p->d_stage.alloc(8 * N))) return rc;
+    // FP64 takes no memory to read v: the residual is scratch between calls and
+    // as large as a field (every node is some element's point)
+    const bool spare = p->prec == SALVUS_FP64 && p->d_r.bytes >= 8 * N;
+    DeviceBuffer &stage = spare ? p->d_r : p->d_stage;
+    if (stage.bytes < 8 * N && (rc = stage.alloc(8 * N))) return rc;
     const unsigned grid = blocks_for((int64_t)N, 256);
     if (!from_w)
       convert_kernel<float, double><<<grid, 256, 0, p->stream>>>((int64_t)N, b->as<float>(),
-                                                                 p->d_stage.as<double>());
+                                                                 stage.as<double>());
     else if (p->prec == SALVUS_FP32)
       velocity_kernel<float><<<grid, 256, 0, p->stream>>>((int64_t)N, b->as<float>(),
                                                           p->d_ap.as<float>(), (float)(0.5 * p->dt),
-                                                          p->d_stage.as<double>());
+                                                          stage.as<double>());
     else
       velocity_kernel<double><<<grid, 256, 0, p->stream>>>((int64_t)N, b->as<double>(),
                                                            p->d_ap.as<double>(), 0.5 * p->dt,
-                                                           p->d_stage.as<double>());
+                                                           stage.as<double>());
     g_launches++;
     if ((rc = check_launch("convert"))) return rc;
-    if ((rc = copy_d2h(p, vals, p->d_stage.ptr, 8 * N))) return rc;
+    if ((rc = copy_d2h(p, vals, stage.ptr, 8 * N))) return rc;
   }
   SALVUS_CUDA(cudaStreamSynchronize(p->stream));
   return device_status(p);
