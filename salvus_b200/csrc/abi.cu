@@ -3145,10 +3145,14 @@ int salvus_get_seismograms(salvus_problem *p, int64_t first, int64_t count, doub
                 (long long)p->seis_cap);
   if (p->recs.empty() || count == 0) return SALVUS_OK;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
-  // The columns asked for, straight into the caller's array (one piece, two
-  // where the window wraps), and the status word, with one wait: copying the
-  // whole ring of 4096 steps and picking from it took 0.1-1.5 ms for what is
-  // 10-50 us (16 to 4096 rows of 16-100 steps, B200).
+  // The columns asked for (one piece, two where the window wraps), not the whole
+  // ring: copying 4096 steps and picking from them took 0.1-1.5 ms for what is
+  // 10-50 us (16 to 4096 rows of 16-100 steps, B200).  The caller's array is
+  // written only if the status is good: windows of up to 32 KB come with the
+  // status word, in one wait, by way of a local buffer; before larger ones the
+  // status is read first (a wait more, about 10 us, where a second copy by the
+  // host would cost more than that).
+  constexpr size_t kLocal = 4096;
   const size_t rows = (size_t)p->shots * p->recs.size() * p->c;
   const int64_t c0 = first % p->seis_cap, n0 = std::min(count, p->seis_cap - c0);
   auto piece = [&](int64_t col, int64_t n, double *to) -> int {
@@ -3157,10 +3161,23 @@ int salvus_get_seismograms(salvus_problem *p, int64_t first, int64_t count, doub
                                   cudaMemcpyDeviceToHost, p->stream));
     return SALVUS_OK;
   };
-  int rc = piece(c0, n0, out);
-  if (rc == SALVUS_OK && n0 < count) rc = piece(0, count - n0, out + n0);
-  if (rc) return rc;
-  return device_status(p);
+  auto window = [&](double *to) -> int {
+    int rc = piece(c0, n0, to);
+    if (rc == SALVUS_OK && n0 < count) rc = piece(0, count - n0, to + n0);
+    return rc;
+  };
+  int rc;
+  if (rows * (size_t)count <= kLocal) {
+    double local[kLocal];
+    rc = window(local);
+    const int done = device_status(p);  // waits for the copies into local too
+    if (rc == SALVUS_OK) rc = done;
+    if (rc == SALVUS_OK) std::memcpy(out, local, sizeof(double) * rows * (size_t)count);
+    return rc;
+  }
+  if ((rc = device_status(p)) || (rc = window(out))) return rc;
+  SALVUS_CUDA(cudaStreamSynchronize(p->stream));
+  return SALVUS_OK;
 }
 
 int salvus_profile_enable(salvus_problem *p, int32_t enable) {

@@ -1,5 +1,6 @@
 """Reading and preparing a problem's state leaves the rest of it alone: no device memory
-is taken to read v of an FP64 problem."""
+is taken to read v of an FP64 problem; a seismogram read that fails leaves the caller's
+array."""
 import numpy as np
 import pytest
 import torch
@@ -36,3 +37,19 @@ def test_reading_v_takes_no_device_memory():
     q.run(5)
     assert np.array_equal(p.get_field("v"), q.get_field("v"))
     assert np.array_equal(p.get_field("u"), q.get_field("u"))
+
+
+@pytest.mark.parametrize("steps", [32, 3000])
+def test_failed_seismogram_read_leaves_the_array(steps):
+    cfg = configs.ricker_2d(nel=6, order=4, n_receivers=16)
+    p = problem(cfg)
+    p.run(steps)
+    want = p.seismograms()
+    bad = np.zeros((p.mesh.n_nodes, 1))
+    bad[p.mesh.n_nodes // 3] = np.nan
+    p.set_field("u", bad)
+    p.run(64)
+    out = np.full(want.shape, 7.0)
+    rc = core.lib().salvus_get_seismograms(p.h, 0, steps, core._dp(out))
+    assert rc == core.E_NONFINITE
+    assert np.all(out == 7.0)
