@@ -1604,6 +1604,7 @@ static int tune_hex(salvus_problem *p) {
   // us a step)
   if (m->order >= 4) {
     p->hex_form = 0;
+    m->hex_wide = 0;  // an earlier problem may have pinned the other
     return SALVUS_OK;
   }
   // problems are prepared on several threads (the job server)
