@@ -920,7 +920,7 @@ static int launch_coupling(salvus_problem *p) {
   const real *coef = sizeof(real) == 4 ? (const real *)m->d_cpl32.ptr : (const real *)m->d_cpl64.ptr;
   coupling_kernel<real><<<blocks_for(m->n_cpl, 256), 256, 0, p->stream>>>(
       m->n_cpl_fluid, m->n_cpl, m->d_cpl_pts.as<int32_t>(), coef, F<real>(p->d_v),
-      F<real>(p->d_ap), (real)(0.5 * p->dt), F<real>(p->d_r));
+      F<real>(p->d_ap), p->half_step ? (real)(0.5 * p->dt) : real(0), F<real>(p->d_r));
   g_launches++;
   return check_launch("coupling");
 }
@@ -2821,7 +2821,6 @@ int salvus_assemble(salvus_problem *p) {
   rc = ready(p);
   if (rc) return rc;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
-  if ((rc = velocity_form(p, true))) return rc;  // the coupling terms read v through w
   if ((rc = sources_ready(p))) return rc;
   return by_components(p->c, [&](auto cc) {
     constexpr int C = decltype(cc)::value;
@@ -3275,8 +3274,10 @@ int salvus_group_run(salvus_group *g, int64_t n_steps) {
   SALVUS_CUDA(cudaSetDevice(g->m0->device));
   for (auto *p : g->members) {
     int rc = ready(p);
-    if (rc || (rc = velocity_form(p, true)) || (rc = sources_ready(p))) return rc;
-    if (!g->stages && n_steps > 0) p->stf_ready = false;  // these forms have no tail
+    if (rc) return rc;
+    if (n_steps == 0) continue;
+    if ((rc = velocity_form(p, true)) || (rc = sources_ready(p))) return rc;
+    if (!g->stages) p->stf_ready = false;  // these forms have no tail
   }
   // order the group after every member's pending work
   for (size_t k = 0; k < g->members.size(); ++k) {

@@ -385,7 +385,7 @@ __global__ void dirichlet_zero_kernel(int64_t n, const int32_t *__restrict__ pts
 // fluid elements (u += cx vx + cy vy), the rest to solid elements
 // (ux += cx v, uy += cy v).  Runs after the stiffness (and Dirichlet zeroing)
 // and before the sources, on the velocity field v = w - dt/2 a_ (these meshes
-// store a_ at every step for it).
+// store a_ at every step for it); hdt = 0: w holds v itself.
 template <typename real>
 __global__ void coupling_kernel(int64_t n_fluid, int64_t n, const int32_t *__restrict__ pts,
                                 const real *__restrict__ coef, const real *__restrict__ w,
@@ -394,7 +394,7 @@ __global__ void coupling_kernel(int64_t n_fluid, int64_t n, const int32_t *__res
   if (i >= n) return;
   const int64_t ep = pts[2 * i], g = pts[2 * i + 1];
   const real cx = coef[2 * i], cy = coef[2 * i + 1];
-  auto v = [&](int64_t x) { return half_step_velocity<real>(w[x], ap[x], hdt); };
+  auto v = [&](int64_t x) { return hdt != 0 ? half_step_velocity<real>(w[x], ap[x], hdt) : w[x]; };
   if (i < n_fluid) {
     r[ep * 3] += cx * v(g * 3 + 1) + cy * v(g * 3 + 2);
   } else {

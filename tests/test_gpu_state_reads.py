@@ -1,6 +1,6 @@
-"""Reading and preparing a problem's state leaves the rest of it alone: no device memory
-is taken to read v of an FP64 problem; a seismogram read that fails leaves the caller's
-array."""
+"""Reading and preparing a problem's state leaves the rest of it alone: fields read back
+as they were set; no device memory is taken to read v of an FP64 problem; a seismogram
+read that fails leaves the caller's array."""
 import numpy as np
 import pytest
 import torch
@@ -17,6 +17,40 @@ def problem(cfg, precision=core.FP32, dt=1.5e-3):
     for r in cfg.get("receivers", []):
         p.add_receiver(r)
     return p
+
+
+@pytest.mark.parametrize("precision", [core.FP32, core.FP64])
+@pytest.mark.parametrize("kind", ["quad", "coupled"])
+def test_assembly_and_empty_runs_keep_the_fields(kind, precision):
+    cfg = (configs.standing_wave_2d(nel=6, order=4) if kind == "quad"
+           else configs.coupled_2d(nel=6, order=3, n_receivers=0))
+    p = problem(cfg, precision)
+    rng = np.random.default_rng(5)
+    shape = (p.mesh.n_nodes, p.c)
+    # a_ far above v / dt: v + dt/2 a_ keeps few digits of v
+    want = {"u": rng.standard_normal(shape), "v": rng.standard_normal(shape),
+            "a_": 1e9 * rng.standard_normal(shape)}
+    if precision == core.FP32:
+        want = {f: x.astype(np.float32).astype(float) for f, x in want.items()}
+    for f, x in want.items():
+        p.set_field(f, x)
+
+    def check():
+        for f, x in want.items():
+            assert np.array_equal(p.get_field(f), x), f
+
+    p.run(0)
+    check()
+    p.assembleIntoGlobalDof()
+    check()
+    p.applyInverseMassMatrix()
+    check()
+    if kind == "quad" and precision == core.FP32:
+        g = core.Group([p])
+        g.run(0)
+        g.synchronize()
+        check()
+        g.close()
 
 
 def test_reading_v_takes_no_device_memory():
