@@ -14,6 +14,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <random>
 #include <thread>
 #include <vector>
@@ -2662,9 +2663,10 @@ static int copy_h2d(salvus_problem *p, void *dst, const void *src, size_t bytes)
 // of the most it replaces about 6.
 static int copy_h2d_f32(salvus_problem *p, float *dst, const double *src, size_t n) {
   if (n * sizeof(float) < 2 * kPinChunk) {
-    std::vector<float> h(n);
-    par_convert(h.data(), src, n);
-    SALVUS_CUDA(cudaMemcpyAsync(dst, h.data(), n * sizeof(float), cudaMemcpyHostToDevice, p->stream));
+    const std::unique_ptr<float[]> h(new (std::nothrow) float[n]);
+    if (!h) return fail(SALVUS_E_OOM, "no host memory for a field of %zu values", n);
+    par_convert(h.get(), src, n);
+    SALVUS_CUDA(cudaMemcpyAsync(dst, h.get(), n * sizeof(float), cudaMemcpyHostToDevice, p->stream));
     SALVUS_CUDA(cudaStreamSynchronize(p->stream));  // the buffer ends here
     return SALVUS_OK;
   }
@@ -2753,9 +2755,7 @@ int salvus_problem_set_field(salvus_problem *p, int32_t f, int32_t shot, const d
   if (!b || shot != 0) return fail(SALVUS_E_INVALID, "bad field %d / shot %d", f, shot);
   const size_t N = (size_t)p->mesh->G * p->c;
   SALVUS_CUDA(cudaSetDevice(p->mesh->device));
-  if (f == SALVUS_FIELD_V) {
-    p->half_step = false;  // v as given; w is formed before the next step
-  } else if (f == SALVUS_FIELD_A_PREV) {
+  if (f == SALVUS_FIELD_A_PREV) {
     if (int rc = velocity_form(p, false)) return rc;  // v does not change with a_
   }
   if (p->prec == SALVUS_FP64) {
@@ -2766,6 +2766,7 @@ int salvus_problem_set_field(salvus_problem *p, int32_t f, int32_t shot, const d
     int rc = copy_h2d_f32(p, b->as<float>(), vals, N);
     if (rc) return rc;
   }
+  if (f == SALVUS_FIELD_V) p->half_step = false;  // v as given; w is formed before the next step
   SALVUS_CUDA(cudaStreamSynchronize(p->stream));
   return SALVUS_OK;
 }

@@ -1,6 +1,12 @@
 """Reading and preparing a problem's state leaves the rest of it alone: fields read back
 as they were set; no device memory is taken to read v of an FP64 problem; a seismogram
-read that fails leaves the caller's array."""
+read that fails leaves the caller's array; a host allocation that fails in set_field is
+an error code."""
+import os
+import subprocess
+import sys
+import textwrap
+
 import numpy as np
 import pytest
 import torch
@@ -8,6 +14,8 @@ import torch
 from salvus_b200 import configs, core
 
 pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def problem(cfg, precision=core.FP32, dt=1.5e-3):
@@ -87,3 +95,41 @@ def test_failed_seismogram_read_leaves_the_array(steps):
     rc = core.lib().salvus_get_seismograms(p.h, 0, steps, core._dp(out))
     assert rc == core.E_NONFINITE
     assert np.all(out == 7.0)
+
+
+def test_set_field_reports_a_failed_host_allocation():
+    """The address space is limited around the call in a process of its own: an
+    error code, not the end of the process; the field is as it was, and the next
+    call works."""
+    code = textwrap.dedent("""
+        import resource
+        import numpy as np
+        from salvus_b200 import configs, core
+        cfg = configs.elastic_hex(nel=34, order=4, n_receivers=0)
+        m = core.Mesh(cfg["shape"], cfg["order"], cfg["physics"], cfg["vertices"], cfg["cells"],
+                      cfg["params"], flags=core.MESH_FP32_ONLY)
+        p = core.Problem(m, core.FP32, dt=1e-4)
+        u = np.random.default_rng(1).standard_normal((m.n_nodes, 3))
+        assert 24 << 20 < 4 * u.size < 64 << 20
+        p.set_field("u", u)
+        p.run(3)
+        v = p.get_field("v")
+        size = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+        hard = resource.getrlimit(resource.RLIMIT_AS)[1]
+        resource.setrlimit(resource.RLIMIT_AS, (size + (8 << 20), hard))
+        try:
+            p.set_field("v", u)
+            raise SystemExit("not refused")
+        except core.SalvusError as e:
+            code = e.code
+        finally:
+            resource.setrlimit(resource.RLIMIT_AS, (hard, hard))
+        assert code == core.E_OOM, code
+        assert np.abs(v).max() > 0 and np.array_equal(p.get_field("v"), v)
+        p.set_field("v", u)
+        assert np.array_equal(p.get_field("v"), u.astype(np.float32))
+        print("refused and went on")
+    """)
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "refused and went on" in r.stdout, r.stdout + r.stderr
