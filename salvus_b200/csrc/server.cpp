@@ -93,6 +93,8 @@ int64_t estimate_bytes(const salvus_mesh_desc &d, int precision) {
   b += E * P * (4 * rw32 + 4 /*conn*/ + 4 /*incidence*/ + 8 /*setup mass, transient*/);
   if (precision == SALVUS_FP64) b += E * P * 8 * rw64;
   b += G * (4 + 8 + 4 + 8 * c);  // offsets, inverse mass, node coordinates
+  if (d.shape == SALVUS_QUAD && d.physics == SALVUS_ACOUSTIC)
+    b += E * P * 4 + E * 16 + G * 8;  // meshes of squares: one number per point; incidence pairs
   b += 4 * G * c * rs;             // u v a a_
   b += E * P * c * rs;             // element-local residual
   b += G * c * 8;                  // host-copy staging
