@@ -913,15 +913,16 @@ static void drop_graph(salvus_problem *p) {
   p->tail_steps = 0;
 }
 
-// fluid-solid coupling integrals (meshes of fluid and solid quadrilaterals)
+// fluid-solid coupling integrals (meshes of fluid and solid quadrilaterals);
+// half_step: what d_v holds when the launch runs (which, captured, is later)
 template <typename real>
-static int launch_coupling(salvus_problem *p) {
+static int launch_coupling(salvus_problem *p, bool half_step) {
   const salvus_mesh *m = p->mesh;
   if (m->physics != SALVUS_COUPLED2D || m->n_cpl == 0) return SALVUS_OK;
   const real *coef = sizeof(real) == 4 ? (const real *)m->d_cpl32.ptr : (const real *)m->d_cpl64.ptr;
   coupling_kernel<real><<<blocks_for(m->n_cpl, 256), 256, 0, p->stream>>>(
       m->n_cpl_fluid, m->n_cpl, m->d_cpl_pts.as<int32_t>(), coef, F<real>(p->d_v),
-      F<real>(p->d_ap), p->half_step ? (real)(0.5 * p->dt) : real(0), F<real>(p->d_r));
+      F<real>(p->d_ap), half_step ? (real)(0.5 * p->dt) : real(0), F<real>(p->d_r));
   g_launches++;
   return check_launch("coupling");
 }
@@ -1105,7 +1106,7 @@ static int step_fused_t(salvus_problem *p, bool store_a) {
   }
   if ((rc = join_receivers(p))) return rc;  // the previous step's receivers
   if ((rc = launch_dirichlet<real, C>(p))) return rc;
-  if ((rc = launch_coupling<real>(p))) return rc;
+  if ((rc = launch_coupling<real>(p, true))) return rc;
   {
     ProfScope ps(p, K_UPDATE);
     if (C == 1 && gather_pairs(m, m->G))
@@ -1439,7 +1440,7 @@ static int assemble_t(salvus_problem *p) {
       return rc;
   }
   if ((rc = launch_dirichlet<real, C>(p))) return rc;
-  if ((rc = launch_coupling<real>(p))) return rc;
+  if ((rc = launch_coupling<real>(p, p->half_step))) return rc;
   ProfScope ps(p, K_GATHER);
   gather_kernel<real, C, 1><<<blocks_for(m->G, 256), 256, 0, p->stream>>>(
       m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), F<real>(p->d_r), nullptr,

@@ -60,6 +60,26 @@ def test_assembly_and_empty_runs_keep_the_fields(kind, precision):
         check()
         g.close()
 
+@pytest.mark.parametrize("precision", [core.FP32, core.FP64])
+@pytest.mark.parametrize("kind", ["quad", "coupled"])
+def test_graphs_captured_before_the_velocity_is_converted(kind, precision):
+    """prepare_run captures while v is as it was set; the run converts it first."""
+    cfg = (configs.standing_wave_2d(nel=6, order=4) if kind == "quad"
+           else configs.coupled_2d(nel=6, order=3, n_receivers=0))
+    got = []
+    for prepare in (False, True):
+        p = problem(cfg, precision)
+        x = np.random.default_rng(6).standard_normal((3, p.mesh.n_nodes, p.c))
+        p.set_field("u", x[0])
+        p.set_field("v", 100.0 * x[1])
+        p.set_field("a_", 1e5 * x[2])
+        if prepare:
+            p.prepare_run(41)
+        p.run(41)
+        got.append([p.get_field(f) for f in ("u", "v", "a_")])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b) and np.isfinite(a).all()
+
 
 def test_reading_v_takes_no_device_memory():
     p = problem(configs.elastic_hex(nel=22, order=4, n_receivers=0), core.FP64, dt=1e-4)
