@@ -202,6 +202,12 @@ class Clocks:
                 "sm_max_mhz": max(mx) if mx else None, "reasons": reasons, "samples": len(rows)}
 
 
+def launch_gaps(ms_per_step, kernels_ms):
+    """What a batched step takes beyond its kernels.  All of them are on its
+    critical path: stiffness, sources, gather and receivers share one stream."""
+    return ms_per_step - sum(kernels_ms.values())
+
+
 def shots_leg(core, configs, timed, steps, n_shots=256, nel=200, device=0):
     """Config 2: n_shots Ricker shots on a nel x nel order-4 quad mesh with a
     seeded smooth velocity model.  Batched form (one graph-replayed launch
@@ -256,8 +262,7 @@ def shots_leg(core, configs, timed, steps, n_shots=256, nel=200, device=0):
             "form": "fused batched step (interior nodes in the stiffness kernel), CUDA graph",
             "shot_throughput_ratio": batched / plain, "steps": steps,
             "kernels_ms": kern,
-            # the receivers overlap the next step's stiffness kernel
-            "launch_gaps_ms_per_step": ms_b / steps - sum(t for k, t in kern.items() if k != "receivers"),
+            "launch_gaps_ms_per_step": launch_gaps(ms_b / steps, kern),
             "tuning": {"stiffness_shot_lanes": tune[0], "stiffness_elements_per_cta": tune[1],
                        "gather_shot_lanes": tune[2], "gather_nodes_per_cta": tune[3]}}
 
