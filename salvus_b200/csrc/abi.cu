@@ -643,20 +643,21 @@ static int incidence_pairs(salvus_mesh *m) {
       total += n > 2 ? n : 0;
     }
   }
-  DeviceBuffer d_base;
+  // base lies behind the lists: freeing a buffer of its own would wait for
+  // everything that other problems have on the device
   int rc;
   if ((rc = m->d_inc_head.alloc(sizeof(int2) * (size_t)m->G)) ||
-      (rc = m->d_inc_rest.alloc(sizeof(int32_t) * (size_t)total)) ||
-      (rc = d_base.alloc(sizeof(int32_t) * base.size())))
+      (rc = m->d_inc_rest.alloc(sizeof(int32_t) * ((size_t)total + base.size()))))
     return rc;
-  SALVUS_CUDA(cudaMemcpyAsync(d_base.ptr, base.data(), sizeof(int32_t) * base.size(),
+  int32_t *rest = m->d_inc_rest.as<int32_t>();
+  SALVUS_CUDA(cudaMemcpyAsync(rest + total, base.data(), sizeof(int32_t) * base.size(),
                               cudaMemcpyHostToDevice, m->stream));
   incidence_pairs_kernel<<<(unsigned)base.size(), kHeadTile, 0, m->stream>>>(
-      m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), d_base.as<int32_t>(),
-      m->d_inc_head.as<int2>(), m->d_inc_rest.as<int32_t>());
+      m->G, m->d_inc_off.as<int32_t>(), m->d_inc_idx.as<int32_t>(), rest + total,
+      m->d_inc_head.as<int2>(), rest);
   g_launches++;
   if ((rc = check_launch("incidence pairs"))) return rc;
-  SALVUS_CUDA(cudaStreamSynchronize(m->stream));  // base and d_base end here
+  SALVUS_CUDA(cudaStreamSynchronize(m->stream));  // base ends here
   return SALVUS_OK;
 }
 

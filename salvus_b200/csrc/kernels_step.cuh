@@ -233,8 +233,7 @@ struct Incidence {
 constexpr int kHeadTile = 256;
 __global__ void __launch_bounds__(kHeadTile)
 incidence_pairs_kernel(int64_t G, const int32_t *__restrict__ off, const int32_t *__restrict__ idx,
-                       const int32_t *__restrict__ base, int2 *__restrict__ head,
-                       int32_t *__restrict__ rest) {
+                       const int32_t *base, int2 *__restrict__ head, int32_t *rest) {
   __shared__ int32_t sum[kHeadTile];
   const int t = threadIdx.x;
   const int64_t g = (int64_t)blockIdx.x * kHeadTile + t;
