@@ -91,13 +91,18 @@ enum salvus_run_mode { SALVUS_RUN_PLAIN = 0, SALVUS_RUN_GRAPH = 1 };
  * constants per point.  Tetrahedra with such material run on CUDA cores;
  * problem groups take isotropic meshes only. */
 #define SALVUS_MESH_ELASTIC_TI 2
-/* salvus_mesh_desc.flags: keep per-point inverse Jacobians for elastic
- * hexahedra even when every element is a parallelepiped.  By default such
- * meshes store one inverse Jacobian per element and FP32 records of the
- * material alone (12 instead of 48 bytes per point with the connectivity);
- * with SALVUS_HEX_STEP=fused in the environment the FP32 step also advances
- * each element's interior nodes inside the stiffness kernel (bitwise the
- * same result; measured slower on the order-4 benchmark mesh). */
+/* salvus_mesh_desc.flags: keep per-point geometry where the elements would
+ * allow less of it.  By default
+ *   elastic hexahedra that are all parallelepipeds store one inverse Jacobian
+ *     per element and records of the material alone (FP32: 12 instead of 48
+ *     bytes per point with the connectivity); FP64 does so only where the
+ *     corners' Jacobians agree to half a rounding of the coordinates, the
+ *     accuracy of a point's own; with SALVUS_HEX_STEP=fused in the environment
+ *     the FP32 step also advances each element's interior nodes inside the
+ *     stiffness kernel (bitwise the same result; slower on every mesh measured);
+ *   acoustic quadrilaterals that are all squares keep one number per point for
+ *     the FP32 single-shot and grouped steps, 8 instead of 16 bytes with the
+ *     node (bitwise the same result). */
 #define SALVUS_MESH_PER_POINT_GEOMETRY 4
 
 typedef struct {
@@ -431,8 +436,12 @@ int salvus_server_destroy(salvus_server *s);
 /* ---- measurement ---- */
 /* Device time of the kernels launched by the last salvus_run / salvus_step
  * calls since the last reset, per kernel class (CUDA events on the problem
- * stream): names[i] (static strings), total_ms[i], launches[i].  Profiling
- * adds an event pair per launch; enable only for measurement. */
+ * stream): names[i] (static strings), total_ms[i], launches[i].  The source
+ * terms of a single-shot step are part of the node gather and their time
+ * functions of the receivers' launch; the sources' own class holds the
+ * evaluation before a first step, the fused hexahedron step's source launch and
+ * that of shot batches.  Profiling adds an event pair per launch; enable only
+ * for measurement. */
 int salvus_profile_enable(salvus_problem *p, int32_t enable);
 int salvus_profile_read(salvus_problem *p, int32_t max_entries, const char **names,
                         double *total_ms, int64_t *launches, int32_t *n_entries);

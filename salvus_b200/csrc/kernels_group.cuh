@@ -264,8 +264,8 @@ group_persistent_step(const GroupSlot *__restrict__ slots, const GroupCounts *__
 // a contiguous range of co-resident CTAs (sized to its share of the group's
 // work) and runs its whole step inside that range: stiffness tiles
 // round-robin over its CTAs; the member's first CTA, once all of them are
-// through the stiffness, adds the sources; after a flag every CTA takes its
-// gather tiles; after all gathers the receivers are spread over the CTAs;
+// through the stiffness, evaluates the source-time functions; after a flag
+// every CTA takes its gather tiles, which add the source terms; after all gathers the receivers are spread over the CTAs;
 // the first CTA then advances the step.  A CTA only ever waits (bounded) for
 // CTAs of its own member, so members never hold each other up, and the
 // cooperative launch guarantees that all CTAs are resident.
