@@ -3161,11 +3161,11 @@ int salvus_get_seismograms(salvus_problem *p, int64_t first, int64_t count, doub
   // The columns asked for (one piece, two where the window wraps), not the whole
   // ring: copying 4096 steps and picking from them took 0.1-1.5 ms for what is
   // 10-50 us (16 to 4096 rows of 16-100 steps, B200).  The caller's array is
-  // written only if the status is good: windows of up to 32 KB come with the
+  // written only if the status is good: windows of up to 128 KB come with the
   // status word, in one wait, by way of a local buffer; before larger ones the
-  // status is read first (a wait more, about 10 us, where a second copy by the
-  // host would cost more than that).
-  constexpr size_t kLocal = 4096;
+  // status is read first (a wait more, 7 us on B200, about what the host takes to
+  // copy 128 KB).
+  constexpr size_t kLocal = 16384;
   const size_t rows = (size_t)p->shots * p->recs.size() * p->c;
   const int64_t c0 = first % p->seis_cap, n0 = std::min(count, p->seis_cap - c0);
   auto piece = [&](int64_t col, int64_t n, double *to) -> int {

@@ -150,6 +150,8 @@ def test_set_field_reports_a_failed_host_allocation():
         assert np.array_equal(p.get_field("v"), u.astype(np.float32))
         print("refused and went on")
     """)
-    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True,
-                       timeout=300)
+    # every large allocation is a mapping of its own, none served from freed memory
+    env = dict(os.environ, MALLOC_MMAP_THRESHOLD_=str(1 << 20))
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True,
+                       text=True, timeout=300)
     assert r.returncode == 0 and "refused and went on" in r.stdout, r.stdout + r.stderr
